@@ -143,8 +143,8 @@ typedef struct myrt_tuning {
   uint32_t trace_persistent; /* 0: one thread per ray; 1: persistent warps that refill finished lanes */
   uint32_t refill;           /* persistent: refill once at least this many lanes of a warp are idle (1..32) */
   uint32_t blocks_per_sm;    /* persistent: resident 128-thread blocks per SM (0 = occupancy maximum) */
-  uint32_t trace_min_blocks; /* one-thread-per-ray: register cap as blocks per SM: 8 (64 regs), 10 (48 regs;
-                                0 = 10), 12 */
+  uint32_t trace_min_blocks; /* one-thread-per-ray: register cap as blocks per SM: 8 (64 regs; 0 = 8),
+                                10 (48 regs), 12 */
   uint32_t trace_unit_steps; /* one-thread-per-ray: 0 = a node and all its triangles per iteration,
                                 1 = one node, triangle or pop per iteration */
   uint32_t wave_paths;       /* physical / guided wavefront: paths in flight per wave (0 = 16 Mi; 4 Mi
@@ -191,8 +191,8 @@ typedef struct myrt_tuning {
                                 1 = grid-stride loops over pt_blocks_per_sm resident blocks per SM,
                                 2 = one thread per queue entry (the grid covers the wave's paths;
                                 blocks past the queue's count return at once; the mesh traversal
-                                kernels then run under a 48-register cap unless pt_blocks_per_sm is
-                                1..9, which gives them 64 registers).
+                                kernels run at 64 registers, or under a 48-register cap when
+                                pt_blocks_per_sm is 10 or more).
                                 Results never depend on it. */
   uint32_t ref_frames;       /* reference shading (myrt_render): frames of one call whose passes run
                                 together, each in its own region of ray slots (0 = as many as fill
@@ -266,7 +266,9 @@ int myrt_trace_any_device(myrt_ctx* ctx, const myrt_ray* rays, uint32_t n, uint8
     void* stream);
 /* Per-ray traversal counters for the closest-hit kernel (device pointers):
  * nodes[i] = wide nodes fetched, tris[i] = triangles tested. Used to count the
- * algorithmic bytes per ray (80 B per node, 48 B per triangle). */
+ * algorithmic bytes per ray (80 B per node, 48 B per triangle). The counted walk
+ * tests child boxes at exactly their quantised planes; the queries widen each
+ * plane by 1/64 of a quantum (trace.cuh), so they may fetch a few more nodes. */
 int myrt_trace_closest_stats_device(myrt_ctx* ctx, const myrt_ray* rays, uint32_t n, myrt_hit* hits,
     uint32_t* nodes, uint32_t* tris, int intersector, void* stream);
 

@@ -264,9 +264,10 @@ int launch_trace_kernels(myrt_ctx* ctx, trace_args a, int intersector, bool any,
     if (rc) return rc;
     return check_cuda(ctx, cudaGetLastError(), "trace launch");
   }
-  // default: the 10-blocks register cap (48 registers, a few bytes of spills),
-  // measured 1 % faster than 8 blocks (64 registers) on 27.9 M-ray batches
-  uint32_t const mb = ctx->tuning.trace_min_blocks ? ctx->tuning.trace_min_blocks : 10u;
+  // default: 8 blocks (64 registers, at most 28 bytes of spills). With the widened planes 10 blocks
+  // (48 registers) spill 84-104 bytes: 27.9 M closest-hit rays 7.60 against 7.09 ms, 3 M watertight
+  // any-hit rays 1.32 against 1.25 ms; 7 and 9 blocks measured 7.16 and 7.39 ms
+  uint32_t const mb = ctx->tuning.trace_min_blocks ? ctx->tuning.trace_min_blocks : 8u;
   bool const unit = ctx->tuning.trace_unit_steps != 0;
   auto go = [&](auto isect_tag) {
     constexpr int IS = decltype(isect_tag)::value;

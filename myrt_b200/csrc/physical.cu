@@ -663,8 +663,9 @@ int launch_plan(myrt_ctx* ctx, physical_state& P, cudaStream_t st, pt_scene cons
     uint32_t const qgrid = per_entry
         ? std::max<uint32_t>(1u, uint32_t((uint64_t(wp.n_paths) + kPtBlock - 1) / kPtBlock))
         : grid;
-    // one thread per entry: the traversal kernels' 10-blocks register cap unless pt_blocks_per_sm is 1..9
-    bool const cap10 = per_entry && (ctx->tuning.pt_blocks_per_sm == 0 || ctx->tuning.pt_blocks_per_sm >= 10);
+    // the mesh traversal kernels at 64 registers; under a 48-register cap (pt_blocks_per_sm >= 10) they
+    // spill 156 bytes: 24.3 against 23.6 ms per 512x512 64-spp frame
+    bool const cap10 = per_entry && ctx->tuning.pt_blocks_per_sm >= 10;
     if (gd) guide_begin_wave(ctx, *gd);
     k_pt_camera<<<grid, kPtBlock, 0, st>>>(w, P.queue[0], P.radiance, P.counts + 0);
     int cur = 0;
