@@ -58,6 +58,16 @@ void free_scene(device_scene& s) {
   s = device_scene{};
 }
 
+void free_sdf(device_sdf& D) {
+  for (void* p : {static_cast<void*>(D.instrs), static_cast<void*>(D.programs), static_cast<void*>(D.params),
+           static_cast<void*>(D.drawables), static_cast<void*>(D.skip_sphere), static_cast<void*>(D.skip_next),
+           static_cast<void*>(D.cell_hdr), static_cast<void*>(D.cell_start), static_cast<void*>(D.cell_list),
+           static_cast<void*>(D.op_count), static_cast<void*>(D.cell_outer), static_cast<void*>(D.chain_hdr), static_cast<void*>(D.chain_rec),
+           static_cast<void*>(D.chain_start), static_cast<void*>(D.chain_list)})
+    cudaFree(p);
+  D = device_sdf{};
+}
+
 bool is_identity(float const* m) {
   for (int c = 0; c < 4; ++c)
     for (int r = 0; r < 4; ++r)
@@ -450,16 +460,7 @@ int myrt_ctx_destroy(myrt_ctx* ctx) {
     if (cs) cudaStreamSynchronize(cs);
   free_scene(ctx->scene);
   ctx->build_scratch.release();
-  cudaFree(ctx->sdf.instrs);
-  cudaFree(ctx->sdf.programs);
-  cudaFree(ctx->sdf.params);
-  cudaFree(ctx->sdf.drawables);
-  cudaFree(ctx->sdf.skip_sphere);
-  cudaFree(ctx->sdf.skip_next);
-  cudaFree(ctx->sdf.cell_hdr);
-  cudaFree(ctx->sdf.cell_start);
-  cudaFree(ctx->sdf.cell_list);
-  cudaFree(ctx->sdf.op_count);
+  free_sdf(ctx->sdf);
   free_render(ctx->render);
   free_textures(ctx);
   free_forward(ctx);
@@ -772,17 +773,7 @@ int myrt_sdf_upload(myrt_ctx* ctx, myrt_sdf_view const* v) {
   if (rc) return rc;
   cudaStreamSynchronize(ctx->stream);
   device_sdf& D = ctx->sdf;
-  cudaFree(D.instrs);
-  cudaFree(D.programs);
-  cudaFree(D.params);
-  cudaFree(D.drawables);
-  cudaFree(D.skip_sphere);
-  cudaFree(D.skip_next);
-  cudaFree(D.cell_hdr);
-  cudaFree(D.cell_start);
-  cudaFree(D.cell_list);
-  cudaFree(D.op_count);
-  D = device_sdf{};
+  free_sdf(D);
   ctx->render.sample_counter = 0;
   if (v->drawable_count == 0) return MYRT_OK;
   if (!v->instrs || !v->programs || !v->drawables || (v->param_count && !v->params))
@@ -831,10 +822,12 @@ int myrt_sdf_upload(myrt_ctx* ctx, myrt_sdf_view const* v) {
   std::vector<int2> skip_next;
   sdf_skip_tables(v, skip_sphere, skip_next);
   sdf_cells cells;
+  sdf_chains chains;
   std::vector<int> op_count;
   if (ctx->tuning.sdf_cells != 1) {
     sdf_cell_tables(v, ctx->tuning.sdf_cells ? int(ctx->tuning.sdf_cells) : 32, cells);
     if (!skip_next.empty() || !cells.list.empty()) sdf_op_counts(v, op_count);
+    sdf_chain_tables(v, cells, chains);
   }
   std::vector<float> dr(v->drawable_count * 36);
   for (size_t d = 0; d < v->drawable_count; ++d) {
@@ -856,6 +849,15 @@ int myrt_sdf_upload(myrt_ctx* ctx, myrt_sdf_view const* v) {
     rc = upload(ctx, &D.cell_hdr, cells.hdr.data(), cells.hdr.size(), "SDF cell headers");
     if (!rc) rc = upload(ctx, &D.cell_start, cells.start.data(), cells.start.size(), "SDF cell starts");
     if (!rc) rc = upload(ctx, &D.cell_list, cells.list.data(), cells.list.size(), "SDF cell lists");
+  }
+  if (!rc && !chains.hdr.empty()) {
+    rc = upload(ctx, &D.cell_outer, cells.outer.data(), cells.outer.size(), "SDF outer grids");
+    if (!rc) rc = upload(ctx, &D.chain_hdr, chains.hdr.data(), chains.hdr.size(), "SDF chain headers");
+    if (!rc) rc = upload(ctx, &D.chain_rec, chains.rec.data(), chains.rec.size(), "SDF chain records");
+    if (!rc) rc = upload(ctx, &D.chain_start, chains.start.data(), chains.start.size(), "SDF chain starts");
+    if (!rc)
+      rc = upload(ctx, &D.chain_list, reinterpret_cast<uint2 const*>(chains.list.data()), chains.list.size() / 4,
+          "SDF chain lists");
   }
   if (!rc && !op_count.empty()) rc = upload(ctx, &D.op_count, op_count.data(), op_count.size(), "SDF operator counts");
   if (!rc) rc = check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "SDF upload");

@@ -82,12 +82,18 @@ struct device_sdf {
   // group's operator, k bits); next 0 = not a skippable group start
   float4* skip_sphere = nullptr;
   int2* skip_next = nullptr;
-  // cell lists of left-to-right chain programs (sdf_skip.hpp sdf_cells),
-  // null when no program has them
+  // cell lists of union-tree programs (sdf_skip.hpp sdf_cells), null when no
+  // program has them
   int4* cell_hdr = nullptr;
   int* cell_start = nullptr;
   uint32_t* cell_list = nullptr;
   int* op_count = nullptr;  // sdf_skip.hpp sdf_op_counts, null when not usable
+  // compiled left folds (sdf_skip.hpp sdf_chain_tables), null when no program is one
+  int4* cell_outer = nullptr;
+  int4* chain_hdr = nullptr;
+  float4* chain_rec = nullptr;
+  int* chain_start = nullptr;
+  uint2* chain_list = nullptr;
   int n_drawables = 0;
   int n_programs = 0;
 };

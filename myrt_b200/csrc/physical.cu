@@ -553,7 +553,8 @@ pt_scene scene_of(myrt_ctx const* ctx) {
       int(S.n_materials), S.material_data, static_cast<ps::area_light const*>(P.lights), P.n_lights,
       sdfk::sdf_dev{ctx->sdf.instrs, ctx->sdf.programs, ctx->sdf.params, ctx->sdf.drawables, ctx->sdf.n_drawables,
           0, 0.f, ctx->sdf.skip_sphere, ctx->sdf.skip_next, ctx->sdf.cell_hdr, ctx->sdf.cell_start,
-          ctx->sdf.cell_list, ctx->sdf.op_count},
+          ctx->sdf.cell_list, ctx->sdf.op_count, ctx->sdf.cell_outer, ctx->sdf.chain_hdr, ctx->sdf.chain_rec, ctx->sdf.chain_start,
+          ctx->sdf.chain_list},
       float3{0.f, 0.f, 0.f}, float3{0.f, 0.f, 0.f}};
   ray_key_grid(S.bounds, r.key_lo, r.key_scale);
   return r;

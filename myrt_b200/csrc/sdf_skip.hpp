@@ -199,12 +199,16 @@ struct sdf_cells {
                                // escape sphere (C.xyz, r_esc) bits
   std::vector<int> start;      // per program (cells + 1) offsets into list
   std::vector<uint32_t> list;  // segment (start | end << 16), relative to the program's first instruction
+  // left folds: a second grid, twice the first one's extent in cells four times
+  // as long, whose cells' offsets and segments follow in start and list
+  std::vector<int4> outer;     // 2 per program: (lo.xyz, 1 / cell) bits; (nx, ny, nz, first cell), nx = 0: none
 };
 
 // cells_long: cells along the grid's longest axis (2..128).
 inline void sdf_cell_tables(myrt_sdf_view const* v, int cells_long, sdf_cells& out) {
   out = sdf_cells{};
   out.hdr.assign(3 * v->program_count, make_int4(0, 0, 0, 0));
+  out.outer.assign(2 * v->program_count, make_int4(0, 0, 0, 0));
   float const* G = v->params;
   struct node {
     int first, end;  // instruction range (end exclusive); an operator's own index is end - 1
@@ -297,122 +301,130 @@ inline void sdf_cell_tables(myrt_sdf_view const* v, int cells_long, sdf_cells& o
       lo_f[a] = float(lo[a]);
       dims[a] = std::max(1, std::min(n_long, int(std::ceil((hi[a] - double(lo_f[a])) * double(inv_f)))));
     }
-    size_t const ncell = size_t(dims[0]) * dims[1] * dims[2];
-    double const cell = 1.0 / double(inv_f);
-    // the device finds a point's cell by rounded float arithmetic: widen each
-    // cell; the margin covers the rounding of every distance and of the
-    // operators' values over the whole program
-    double const widen = 1e-4 * cell + 1e-6 * scale;
-    double const margin = 2e-3 + 4e-6 * double(n_prims) * scale;
-    size_t const first_start = out.start.size();
-    size_t const first_entry = out.list.size();
+    // Appends the cell lists of one grid to out.start / out.list. False when
+    // they would take too many entries.
     // z-slabs of cells on host threads; each keeps its cells' segment counts
     // and segments, concatenated in cell order afterwards
-    struct slab {
-      std::vector<int> sizes;
-      std::vector<uint32_t> segs;
-    };
-    int const n_threads = std::max(1, std::min<int>(dims[2], int(std::thread::hardware_concurrency())));
-    std::vector<slab> slabs(n_threads);
-    auto fill = [&](int t) {
-      slab& out_t = slabs[t];
-      std::vector<double> lb(ns.size()), ub(ns.size());
-      std::vector<int> todo;
-      uint32_t seg_s = 0, seg_e = 0;
-      bool open = false;
-      auto exec = [&](int s0, int e0) {  // append [s0, e0), merging with the open segment
-        if (open && int(seg_e) == s0) {
-          seg_e = uint32_t(e0);
-          return;
-        }
-        if (open) out_t.segs.push_back(seg_s | (seg_e << 16));
-        seg_s = uint32_t(s0);
-        seg_e = uint32_t(e0);
-        open = true;
+    auto add_grid = [&](float const (&lo_f)[3], float inv_f, int const (&dims)[3], double scale) -> bool {
+      size_t const ncell = size_t(dims[0]) * dims[1] * dims[2];
+      double const cell = 1.0 / double(inv_f);
+      // the device finds a point's cell by rounded float arithmetic: widen each
+      // cell; the margin covers the rounding of every distance and of the
+      // operators' values over the whole program
+      double const widen = 1e-4 * cell + 1e-6 * scale;
+      double const margin = 2e-3 + 4e-6 * double(n_prims) * scale;
+      size_t const first_start = out.start.size();
+      size_t const first_entry = out.list.size();
+      struct slab {
+        std::vector<int> sizes;
+        std::vector<uint32_t> segs;
       };
-      int const z0 = int(int64_t(dims[2]) * t / n_threads), z1 = int(int64_t(dims[2]) * (t + 1) / n_threads);
-      for (int z = z0; z < z1; ++z)
-        for (int y = 0; y < dims[1]; ++y)
-          for (int x = 0; x < dims[0]; ++x) {
-            int const idx[3] = {x, y, z};
-            double bmin[3], bmax[3];
-            for (int a = 0; a < 3; ++a) {
-              bmin[a] = double(lo_f[a]) + idx[a] * cell - widen;
-              bmax[a] = double(lo_f[a]) + (idx[a] + 1) * cell + widen;
-            }
-            size_t const before = out_t.segs.size();
-            for (size_t i = 0; i < ns.size(); ++i) {  // operands come before their operator
-              node const& n = ns[i];
-              if (n.a < 0) {
-                double n2 = 0.0, f2 = 0.0;
-                for (int a = 0; a < 3; ++a) {
-                  double const o = std::fmax(0.0, std::fmax(bmin[a] - n.c[a], n.c[a] - bmax[a]));
-                  double const f = std::fmax(std::fabs(n.c[a] - bmin[a]), std::fabs(n.c[a] - bmax[a]));
-                  n2 += o * o;
-                  f2 += f * f;
-                }
-                lb[i] = std::sqrt(n2) - n.R;
-                ub[i] = std::sqrt(f2) + n.U;
-              } else {
-                // lb of an operator node is (its primitives' smallest bound -
-                // its delta); lb + delta recovers the primitives' bound
-                lb[i] = std::fmin(lb[n.a] + ns[n.a].delta, lb[n.b] + ns[n.b].delta) - n.delta;
-                ub[i] = std::fmin(ub[n.a], ub[n.b]);
-              }
-            }
-            open = false;
-            todo.assign(1, root);
-            while (!todo.empty()) {  // depth first, left operand first
-              int const i = todo.back();
-              todo.pop_back();
-              if (i < 0) {  // an operator kept with both operands
-                exec(-i - 1, -i);
-                continue;
-              }
-              node const& n = ns[i];
-              if (n.a < 0) {
-                exec(n.first, n.end);
-                continue;
-              }
-              if (lb[n.b] >= ub[n.a] + n.k + margin) {
-                todo.push_back(n.a);  // the right operand and the operator drop out
-              } else if (lb[n.a] >= ub[n.b] + n.k + margin) {
-                todo.push_back(n.b);  // the left operand and the operator drop out
-              } else {
-                todo.push_back(-(n.end - 1) - 1);
-                todo.push_back(n.b);
-                todo.push_back(n.a);
-              }
-            }
-            if (open) out_t.segs.push_back(seg_s | (seg_e << 16));
-            out_t.sizes.push_back(int(out_t.segs.size() - before));
+      int const n_threads = std::max(1, std::min<int>(dims[2], int(std::thread::hardware_concurrency())));
+      std::vector<slab> slabs(n_threads);
+      auto fill = [&](int t) {
+        slab& out_t = slabs[t];
+        std::vector<double> lb(ns.size()), ub(ns.size());
+        std::vector<int> todo;
+        uint32_t seg_s = 0, seg_e = 0;
+        bool open = false;
+        auto exec = [&](int s0, int e0) {  // append [s0, e0), merging with the open segment
+          if (open && int(seg_e) == s0) {
+            seg_e = uint32_t(e0);
+            return;
           }
-    };
-    {
-      std::vector<std::thread> pool;
-      for (int t = 1; t < n_threads; ++t) pool.emplace_back(fill, t);
-      fill(0);
-      for (std::thread& th : pool) th.join();
-    }
-    size_t total = out.list.size();
-    for (slab const& sl : slabs) total += sl.segs.size();
-    if (total > max_entries) continue;  // too large: no cells for this program
-    out.start.reserve(first_start + ncell + 1);
-    out.list.reserve(total);
-    for (slab const& sl : slabs) {
-      for (int n_seg : sl.sizes) {
-        out.start.push_back(int(out.list.size()));
-        out.list.resize(out.list.size() + size_t(n_seg));
+          if (open) out_t.segs.push_back(seg_s | (seg_e << 16));
+          seg_s = uint32_t(s0);
+          seg_e = uint32_t(e0);
+          open = true;
+        };
+        int const z0 = int(int64_t(dims[2]) * t / n_threads), z1 = int(int64_t(dims[2]) * (t + 1) / n_threads);
+        for (int z = z0; z < z1; ++z)
+          for (int y = 0; y < dims[1]; ++y)
+            for (int x = 0; x < dims[0]; ++x) {
+              int const idx[3] = {x, y, z};
+              double bmin[3], bmax[3];
+              for (int a = 0; a < 3; ++a) {
+                bmin[a] = double(lo_f[a]) + idx[a] * cell - widen;
+                bmax[a] = double(lo_f[a]) + (idx[a] + 1) * cell + widen;
+              }
+              size_t const before = out_t.segs.size();
+              for (size_t i = 0; i < ns.size(); ++i) {  // operands come before their operator
+                node const& n = ns[i];
+                if (n.a < 0) {
+                  double n2 = 0.0, f2 = 0.0;
+                  for (int a = 0; a < 3; ++a) {
+                    double const o = std::fmax(0.0, std::fmax(bmin[a] - n.c[a], n.c[a] - bmax[a]));
+                    double const f = std::fmax(std::fabs(n.c[a] - bmin[a]), std::fabs(n.c[a] - bmax[a]));
+                    n2 += o * o;
+                    f2 += f * f;
+                  }
+                  lb[i] = std::sqrt(n2) - n.R;
+                  ub[i] = std::sqrt(f2) + n.U;
+                } else {
+                  // lb of an operator node is (its primitives' smallest bound -
+                  // its delta); lb + delta recovers the primitives' bound
+                  lb[i] = std::fmin(lb[n.a] + ns[n.a].delta, lb[n.b] + ns[n.b].delta) - n.delta;
+                  ub[i] = std::fmin(ub[n.a], ub[n.b]);
+                }
+              }
+              open = false;
+              todo.assign(1, root);
+              while (!todo.empty()) {  // depth first, left operand first
+                int const i = todo.back();
+                todo.pop_back();
+                if (i < 0) {  // an operator kept with both operands
+                  exec(-i - 1, -i);
+                  continue;
+                }
+                node const& n = ns[i];
+                if (n.a < 0) {
+                  exec(n.first, n.end);
+                  continue;
+                }
+                if (lb[n.b] >= ub[n.a] + n.k + margin) {
+                  todo.push_back(n.a);  // the right operand and the operator drop out
+                } else if (lb[n.a] >= ub[n.b] + n.k + margin) {
+                  todo.push_back(n.b);  // the left operand and the operator drop out
+                } else {
+                  todo.push_back(-(n.end - 1) - 1);
+                  todo.push_back(n.b);
+                  todo.push_back(n.a);
+                }
+              }
+              if (open) out_t.segs.push_back(seg_s | (seg_e << 16));
+              out_t.sizes.push_back(int(out_t.segs.size() - before));
+            }
+      };
+      {
+        std::vector<std::thread> pool;
+        for (int t = 1; t < n_threads; ++t) pool.emplace_back(fill, t);
+        fill(0);
+        for (std::thread& th : pool) th.join();
       }
-    }
-    {  // copy the segments behind the offsets just laid out
-      size_t at = first_entry;
+      size_t total = out.list.size();
+      for (slab const& sl : slabs) total += sl.segs.size();
+      if (total > max_entries) return false;
+      out.start.reserve(first_start + ncell + 1);
+      out.list.reserve(total);
       for (slab const& sl : slabs) {
-        std::copy(sl.segs.begin(), sl.segs.end(), out.list.begin() + ptrdiff_t(at));
-        at += sl.segs.size();
+        for (int n_seg : sl.sizes) {
+          out.start.push_back(int(out.list.size()));
+          out.list.resize(out.list.size() + size_t(n_seg));
+        }
       }
-    }
-    out.start.push_back(int(out.list.size()));
+      {  // copy the segments behind the offsets just laid out
+        size_t at = first_entry;
+        for (slab const& sl : slabs) {
+          std::copy(sl.segs.begin(), sl.segs.end(), out.list.begin() + ptrdiff_t(at));
+          at += sl.segs.size();
+        }
+      }
+      out.start.push_back(int(out.list.size()));
+      return true;
+    };
+    size_t const first_start = out.start.size();
+    if (!add_grid(lo_f, inv_f, dims, scale)) continue;  // too large: no cells for this program
+    double const margin = 2e-3 + 4e-6 * double(n_prims) * scale;
     // escape sphere about the grid's centre; the radius carries a relative
     // margin for the rounding of values and positions far from the field
     float esc[4];
@@ -432,8 +444,146 @@ inline void sdf_cell_tables(myrt_sdf_view const* v, int cells_long, sdf_cells& o
     out.hdr[3 * p + 1] = make_int4(dims[0], dims[1], dims[2], int(first_start));
     out.hdr[3 * p + 2] = make_int4(esc_bits[0], esc_bits[1], esc_bits[2], esc_bits[3]);
     any = true;
+    bool fold = true;  // every operator's right operand is a primitive
+    for (node const& n : ns) fold = fold && (n.a < 0 || ns[n.b].a < 0);
+    if (!fold) continue;
+    float const inv2 = 0.25f * inv_f;
+    float lo2[3];
+    int dims2[3];
+    double scale2 = scale;
+    for (int a = 0; a < 3; ++a) {
+      double const half = 0.5 * double(dims[a]) / double(inv_f), mid = double(lo_f[a]) + half;
+      lo2[a] = float(mid - 2.0 * half);
+      dims2[a] = std::max(1, (2 * dims[a] + 3) / 4);
+      scale2 = std::fmax(scale2, std::fabs(mid) + 2.0 * half + 4.0 / double(inv_f));
+    }
+    size_t const outer_start = out.start.size();
+    if (!add_grid(lo2, inv2, dims2, scale2)) continue;
+    int lo2_bits[3], inv2_bits;
+    std::memcpy(lo2_bits, lo2, sizeof lo2_bits);
+    std::memcpy(&inv2_bits, &inv2, sizeof inv2_bits);
+    out.outer[2 * p + 0] = make_int4(lo2_bits[0], lo2_bits[1], lo2_bits[2], inv2_bits);
+    out.outer[2 * p + 1] = make_int4(dims2[0], dims2[1], dims2[2], int(outer_start));
   }
   if (!any) out = sdf_cells{};
+}
+
+// Compiled left folds. A program that folds bounded primitives from left to
+// right -- group 0: [translate] primitive, group g: [translate] primitive,
+// union / smooth union -- and has cell lists is also kept as one record per
+// group, and each cell's segments as the list of its groups, so that the
+// evaluator (sdf.cuh chain_map) runs without decoding instructions and without
+// a stack. Record (3 float4): bounding sphere (c, R + k) of the group, as
+// sdf_skip_tables; (offset.xyz, kind bits: primitive op | 256 for a union);
+// (primitive parameters, k). One more record ends the program's: a sphere of
+// radius -inf, skipped at every point, which fills lists up to four entries.
+struct sdf_chains {
+  std::vector<int4> hdr;        // per program: (first record, groups, full list's first and end batch); groups 0: none
+  std::vector<float4> rec;      // 3 per group
+  std::vector<int> start;       // parallel to sdf_cells::start: first batch of four entries
+  std::vector<uint16_t> list;   // group numbers, lists padded to whole batches with the program's last record
+};
+
+inline void sdf_chain_tables(myrt_sdf_view const* v, sdf_cells const& cells, sdf_chains& out) {
+  out = sdf_chains{};
+  if (cells.list.empty()) return;
+  out.hdr.assign(v->program_count, make_int4(0, 0, 0, 0));
+  out.start.assign(cells.start.size(), 0);
+  float const* G = v->params;
+  bool any = false;
+  auto bits = [](int i) {
+    float f;
+    std::memcpy(&f, &i, sizeof f);
+    return f;
+  };
+  for (size_t p = 0; p < v->program_count; ++p) {
+    int4 const dims = cells.hdr[3 * p + 1];
+    if (dims.x <= 0) continue;
+    myrt_sdf_program const pr = v->programs[p];
+    std::vector<float4> rec;
+    std::vector<int> group(pr.count, -1);    // instruction -> its group
+    std::vector<uint8_t> is_op(pr.count, 0);
+    bool ok = true;
+    int g = 0;
+    for (int j = 0; ok && j < pr.count; ++g) {
+      float off[3] = {0.f, 0.f, 0.f};
+      myrt_sdf_instr in = v->instrs[pr.first + j];
+      if (in.op == MYRT_SDF_TRANSLATE) {  // one translation at most: p - 0 is p, two would round twice
+        std::memcpy(off, G + in.param_offset, sizeof off);
+        group[j++] = g;
+        if (j >= pr.count) { ok = false; break; }
+        in = v->instrs[pr.first + j];
+      }
+      double c[3] = {off[0], off[1], off[2]}, R = 0.0, U = 0.0;
+      float const* q = G + in.param_offset;
+      if (!sdf_prim_bounds(in.op, q, c, R, U)) { ok = false; break; }
+      group[j++] = g;
+      int kind = in.op;
+      float k = 0.f;
+      if (g > 0) {
+        if (j >= pr.count) { ok = false; break; }
+        myrt_sdf_instr const op = v->instrs[pr.first + j];
+        if (op.op == MYRT_SDF_UNION) kind |= 256;
+        else if (op.op == MYRT_SDF_SMOOTH_UNION && G[op.param_offset] > 0.f) k = G[op.param_offset];
+        else { ok = false; break; }
+        is_op[j] = 1;
+        group[j++] = g;
+      }
+      float const Rf = float(R) + 1e-6f * float(std::fabs(R));
+      rec.push_back(make_float4(float(c[0]), float(c[1]), float(c[2]), Rf + k));
+      rec.push_back(make_float4(off[0], off[1], off[2], bits(kind)));
+      bool const box = in.op == MYRT_SDF_BOX;
+      rec.push_back(make_float4(q[0], in.op == MYRT_SDF_SPHERE ? 0.f : q[1], box ? q[2] : 0.f, k));
+    }
+    if (!ok || g < 2 || g >= 65535) continue;
+    // the cells' groups (both grids), and every group as one more list
+    std::vector<uint16_t> list;
+    auto close = [&] {
+      while (list.size() & 3u) list.push_back(uint16_t(g));
+    };
+    int const base = int(out.list.size() / 4);
+    for (int4 const grid : {dims, cells.outer[2 * p + 1]}) {
+      size_t const ncell = size_t(grid.x) * grid.y * grid.z;
+      for (size_t c = 0; ok && c < ncell; ++c) {
+        out.start[grid.w + c] = base + int(list.size() / 4);
+        int last = -1;
+        for (int e = cells.start[grid.w + c]; ok && e < cells.start[grid.w + c + 1]; ++e) {
+          int const s0 = int(cells.list[e] & 0xffffu), s1 = int(cells.list[e] >> 16);
+          for (int j = s0; j < s1; ++j) {
+            if (is_op[j]) {
+              ok = ok && group[j] == last;  // an operator follows its own group's primitive
+              continue;
+            }
+            if (group[j] == last) continue;  // translation, then primitive
+            // a group after the list's first needs its operator in the same segment
+            bool const first_of_list = last < 0;
+            last = group[j];
+            int end = j;
+            while (end < s1 && group[end] == last) ++end;
+            ok = ok && first_of_list != bool(is_op[end - 1]);
+            list.push_back(uint16_t(last));
+          }
+        }
+        ok = ok && last >= 0;
+        close();
+      }
+      if (ncell) out.start[grid.w + ncell] = base + int(list.size() / 4);
+    }
+    if (!ok || list.size() / 4 + out.list.size() / 4 > (size_t(1) << 28)) continue;
+    out.list.insert(out.list.end(), list.begin(), list.end());
+    list.clear();
+    for (int k = 0; k < g; ++k) list.push_back(uint16_t(k));
+    close();
+    int const full = int(out.list.size() / 4);
+    out.list.insert(out.list.end(), list.begin(), list.end());
+    out.hdr[p] = make_int4(int(out.rec.size() / 3), g, full, int(out.list.size() / 4));
+    rec.push_back(make_float4(0.f, 0.f, 0.f, -HUGE_VALF));
+    rec.push_back(make_float4(0.f, 0.f, 0.f, bits(MYRT_SDF_SPHERE)));
+    rec.push_back(make_float4(0.f, 0.f, 0.f, 1.f));
+    out.rec.insert(out.rec.end(), rec.begin(), rec.end());
+    any = true;
+  }
+  if (!any) out = sdf_chains{};
 }
 
 }  // namespace myrt_b200
