@@ -15,12 +15,12 @@
 //   k_radix_tree   binary radix tree over the sorted codes (Karras, "Maximizing
 //                  parallelism in the construction of BVHs, octrees and k-d
 //                  trees", HPG 2012); equal codes are ordered by position
-//   k_boxes_up     internal boxes bottom-up, the second child to arrive at a
-//                  node computes its box (atomic arrival counters)
-//   k_collapse     one wide node per thread, level by level: expand the
+//   k_boxes_block, k_boxes_cross  internal boxes, as ranges of leaf boxes
+//   k_collapse     one wide node per 8 lanes, level by level: expand the
 //                  largest-area child with more than 4 triangles until 8
 //                  children, then quantise, assign slots by octant and emit
-//                  the node, its triangles and its internal children
+//                  the node, its triangles' prims and its internal children
+//   k_emit_tris    the leaf-ordered triangles
 #include <cuda_runtime.h>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -37,8 +37,11 @@ namespace myrt_b200 {
 namespace {
 
 constexpr uint32_t kLeafBit = 0x80000000u;
-constexpr uint32_t kNone = 0xffffffffu;
+constexpr uint32_t kNone = 0xffffffffu;  // no node
 constexpr int kMaxLeaf = 4;
+constexpr int kMaxLevels = 4096;
+constexpr uint32_t kColGrid = 2368;   // collapse blocks of a large level: 16 for each of 148 SMs
+constexpr uint32_t kCrossGrid = 592;  // blocks of k_boxes_cross: 4 for each of 148 SMs
 
 struct ibox {
   float4 lo, hi;  // w unused
@@ -116,9 +119,9 @@ __device__ __forceinline__ int delta(uint64_t const* k, int n, int i, int j) {
   return __clzll(a ^ b);
 }
 
-// internal node i: children (leaf bit | index), prim range, parents
+// internal node i: children (leaf bit | index), prim range
 __global__ void k_radix_tree(uint64_t const* __restrict__ keys, int n, uint2* __restrict__ child,
-    uint2* __restrict__ range, uint32_t* __restrict__ parent_internal, uint32_t* __restrict__ parent_leaf) {
+    uint2* __restrict__ range) {
   int const i = int(blockIdx.x * blockDim.x + threadIdx.x);
   if (i >= n - 1) return;
   int const d = (delta(keys, n, i, i + 1) - delta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
@@ -142,18 +145,14 @@ __global__ void k_radix_tree(uint64_t const* __restrict__ keys, int n, uint2* __
   uint32_t const right = last == gamma + 1 ? (kLeafBit | uint32_t(gamma + 1)) : uint32_t(gamma + 1);
   child[i] = make_uint2(left, right);
   range[i] = make_uint2(uint32_t(first), uint32_t(last));
-  if (left & kLeafBit) parent_leaf[gamma] = uint32_t(i);
-  else parent_internal[gamma] = uint32_t(i);
-  if (right & kLeafBit) parent_leaf[gamma + 1] = uint32_t(i);
-  else parent_internal[gamma + 1] = uint32_t(i);
 }
 
 __device__ __forceinline__ ibox load_box(uint32_t ref, ibox const* leaf_boxes, uint32_t const* order,
     ibox const* inner) {
   if (ref & kLeafBit) return leaf_boxes[order[ref & ~kLeafBit]];
   ibox b;
-  b.lo = __ldcg(&inner[ref].lo);
-  b.hi = __ldcg(&inner[ref].hi);
+  b.lo = inner[ref].lo;
+  b.hi = inner[ref].hi;
   return b;
 }
 __device__ __forceinline__ ibox merge(ibox a, ibox b) {
@@ -161,20 +160,74 @@ __device__ __forceinline__ ibox merge(ibox a, ibox b) {
       make_float4(fmaxf(a.hi.x, b.hi.x), fmaxf(a.hi.y, b.hi.y), fmaxf(a.hi.z, b.hi.z), 0.f)};
 }
 
-__global__ void k_boxes_up(ibox const* __restrict__ leaf_boxes, uint32_t const* __restrict__ order, int n,
-    uint2 const* __restrict__ child, uint32_t const* __restrict__ parent_internal,
-    uint32_t const* __restrict__ parent_leaf, uint32_t* __restrict__ arrivals, ibox* __restrict__ inner) {
-  int const l = int(blockIdx.x * blockDim.x + threadIdx.x);
-  if (l >= n || n < 2) return;
-  uint32_t node = parent_leaf[l];
-  while (node != kNone) {
-    __threadfence();
-    if (atomicAdd(&arrivals[node], 1u) == 0u) return;  // the sibling is not done yet
-    uint2 const c = child[node];
-    ibox const b = merge(load_box(c.x, leaf_boxes, order, inner), load_box(c.y, leaf_boxes, order, inner));
-    __stcg(&inner[node].lo, b.lo);
-    __stcg(&inner[node].hi, b.hi);
-    node = parent_internal[node];
+// Boxes of the internal nodes. A node covers a range of the sorted leaves, so
+// its box is a range minimum / maximum over leaf boxes: no order among nodes,
+// where a bottom-up pass is a chain of global arrivals, fences and loads as
+// long as the tree is deep (655,872 triangles: 81 us; 96 us with the lower
+// levels' arrivals in shared memory). k_boxes_block keeps the boxes of every
+// run of 2^j leaves of its 256 (eight levels, 48 KB) and answers each node
+// within them from two runs; it also writes the 256 leaves' own box and lists
+// the nodes that reach past them. k_boxes_cross gives each of those a warp:
+// the leaves at both ends and the whole blocks between. Together 50 us.
+constexpr int kBoxBlock = 256, kBoxRuns = 8;
+__global__ void __launch_bounds__(kBoxBlock) k_boxes_block(ibox const* __restrict__ leaf_boxes,
+    uint32_t const* __restrict__ order, int n, uint2 const* __restrict__ range, ibox* __restrict__ inner,
+    ibox* __restrict__ block_box, uint32_t* __restrict__ cross, uint32_t* __restrict__ n_cross) {
+  __shared__ float s_run[kBoxRuns][6][kBoxBlock];
+  uint32_t const b0 = blockIdx.x * kBoxBlock, t = threadIdx.x;
+  bool const leaf = b0 + t < uint32_t(n);
+  float v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  if (leaf) {
+    ibox const b = leaf_boxes[order[b0 + t]];
+    v[0] = b.lo.x, v[1] = b.lo.y, v[2] = b.lo.z, v[3] = b.hi.x, v[4] = b.hi.y, v[5] = b.hi.z;
+  }
+#pragma unroll
+  for (int j = 0; j < kBoxRuns; ++j) {  // s_run[j][.][t]: leaves t .. t + 2^j - 1 (those of the block)
+    if (j > 0) {
+      uint32_t const o = t + (1u << (j - 1));
+      if (o < kBoxBlock)
+        for (int c = 0; c < 6; ++c)
+          v[c] = c < 3 ? fminf(v[c], s_run[j - 1][c][o]) : fmaxf(v[c], s_run[j - 1][c][o]);
+    }
+    for (int c = 0; c < 6; ++c) s_run[j][c][t] = v[c];
+    __syncthreads();
+  }
+  auto runs = [&](uint32_t lo, uint32_t hi) {  // leaves lo .. hi of the block
+    int const j = min(31 - __clz(hi - lo + 1u), kBoxRuns - 1);
+    uint32_t const o = hi + 1u - (1u << j);
+    float w[6];
+    for (int c = 0; c < 6; ++c)
+      w[c] = c < 3 ? fminf(s_run[j][c][lo], s_run[j][c][o]) : fmaxf(s_run[j][c][lo], s_run[j][c][o]);
+    return ibox{make_float4(w[0], w[1], w[2], 0.f), make_float4(w[3], w[4], w[5], 0.f)};
+  };
+  if (t == 0) block_box[blockIdx.x] = runs(0u, kBoxBlock - 1u);
+  if (b0 + t >= uint32_t(n) - 1u) return;  // n - 1 internal nodes
+  uint2 const r = range[b0 + t];
+  if (r.x >= b0 && r.y < b0 + kBoxBlock) inner[b0 + t] = runs(r.x - b0, r.y - b0);
+  else cross[atomicAdd(n_cross, 1u)] = b0 + t;
+}
+
+__global__ void __launch_bounds__(256) k_boxes_cross(ibox const* __restrict__ leaf_boxes,
+    uint32_t const* __restrict__ order, uint2 const* __restrict__ range, ibox const* __restrict__ block_box,
+    uint32_t const* __restrict__ cross, uint32_t const* __restrict__ n_cross, ibox* __restrict__ inner) {
+  uint32_t const lane = threadIdx.x & 31u, n = *n_cross;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
+    uint32_t const node = cross[i];
+    uint2 const r = range[node];
+    uint32_t const bx = r.x / kBoxBlock, by = r.y / kBoxBlock;  // bx < by
+    ibox b{make_float4(INFINITY, INFINITY, INFINITY, 0.f), make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f)};
+    for (uint32_t l = r.x + lane; l < (bx + 1u) * kBoxBlock; l += 32u) b = merge(b, leaf_boxes[order[l]]);
+    for (uint32_t l = by * kBoxBlock + lane; l <= r.y; l += 32u) b = merge(b, leaf_boxes[order[l]]);
+    for (uint32_t k = bx + 1u + lane; k < by; k += 32u) b = merge(b, block_box[k]);
+    float* const f[6] = {&b.lo.x, &b.lo.y, &b.lo.z, &b.hi.x, &b.hi.y, &b.hi.z};
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int c = 0; c < 6; ++c) {
+        float const v = __shfl_xor_sync(0xffffffffu, *f[c], o);
+        *f[c] = c < 3 ? fminf(*f[c], v) : fmaxf(*f[c], v);
+      }
+    if (lane == 0) inner[node] = b;
   }
 }
 
@@ -190,15 +243,13 @@ struct collapse_args {
   uint2 const* child;
   uint2 const* range;
   ibox const* inner;
-  float const* pos;        // world triangles, 9 floats per prim
   bvh8_node* nodes;
-  float4* tris;            // 3 per triangle
-  uint32_t* counters;      // [0] wide nodes, [1] triangles, [2] / [5] queue lengths, [3] max depth, [4] leaf slots
+  uint32_t* tri_prim;      // leaf-ordered triangle -> prim
+  uint32_t* counters;      // [0] wide nodes, [1] triangles, [3] max depth, [4] leaf slots
   collapse_item const* in;
   uint32_t const* n_in;    // this level's queue length (device)
   collapse_item* out;
-  uint32_t* n_out;         // the next level's (zeroed before the launch)
-  int n;
+  uint32_t* n_out;         // the next level's (zeroed before the build)
 };
 
 __device__ __forceinline__ uint32_t prim_count(collapse_args const& a, uint32_t ref) {
@@ -206,171 +257,246 @@ __device__ __forceinline__ uint32_t prim_count(collapse_args const& a, uint32_t 
   uint2 const r = a.range[ref];
   return r.y - r.x + 1u;
 }
-__device__ __forceinline__ uint2 prim_range(collapse_args const& a, uint32_t ref) {
-  if (ref & kLeafBit) return make_uint2(ref & ~kLeafBit, ref & ~kLeafBit);
-  return a.range[ref];
-}
 __device__ __forceinline__ float area(ibox const& b) {
   float const dx = b.hi.x - b.lo.x, dy = b.hi.y - b.lo.y, dz = b.hi.z - b.lo.z;
   return ((dx + dy) * dz + dx * dy) * 2.f;
 }
 
+// 2^e as a double, -1022 <= e <= 1023
+__device__ __forceinline__ double pow2(int e) { return __longlong_as_double(static_cast<long long>(1023 + e) << 52); }
+
 // Smallest e with extent / 2^e <= 255 (the host builder's biased_exponent_for).
 __device__ __forceinline__ uint8_t biased_exponent(float extent) {
   if (!(extent > 0.f)) return uint8_t(127 - 100);
-  int e;
-  frexp(double(extent) / 255.0, &e);  // extent / 255 = m 2^e, m in [0.5, 1)
-  while (e > -126 && ldexp(255.0, e - 1) >= double(extent)) --e;
-  while (ldexp(255.0, e) < double(extent)) ++e;
+  // extent / 255 in [2^(e-1), 2^e); its rounding can put it one binade off
+  int e = int((__double_as_longlong(double(extent) / 255.0) >> 52) & 0x7ff) - 1022;
+  while (e > -126 && 255.0 * pow2(e - 1) >= double(extent)) --e;
+  while (255.0 * pow2(e) < double(extent)) ++e;
   e = max(-126, min(127, e));
   return uint8_t(e + 127);
 }
 
-__global__ void k_collapse(collapse_args a) {
-  uint32_t const it = blockIdx.x * blockDim.x + threadIdx.x;
-  if (it >= *a.n_in) return;
-  collapse_item const item = a.in[it];
-  uint32_t kids[8];
-  ibox kb[8];
-  int nk = 0;
-  if ((item.ref & kLeafBit) || prim_count(a, item.ref) <= uint32_t(kMaxLeaf)) {
-    kids[0] = item.ref;  // the whole (small) tree is one leaf slot
-    nk = 1;
-  } else {
-    uint2 const c = a.child[item.ref];
-    kids[0] = c.x;
-    kids[1] = c.y;
-    nk = 2;
-    while (nk < 8) {
-      int best = -1;
-      float ba = -1.f;
-      for (int k = 0; k < nk; ++k) {
-        if ((kids[k] & kLeafBit) || prim_count(a, kids[k]) <= uint32_t(kMaxLeaf)) continue;
-        float const ar = area(load_box(kids[k], a.leaf_boxes, a.order, a.inner));
-        if (ar > ba) {
-          ba = ar;
-          best = k;
-        }
+// One wide node per 8 lanes of a warp, lane k holding child k while the node
+// is opened and slot k once the slots are assigned. A level of the tree is one
+// launch and its time was the serial work of one thread -- 7 dependent
+// expansions, a 64-entry cost search per slot, 24 double divisions, calls of
+// frexp and ldexp -- on arrays in local memory; spread over 8 lanes the search
+// and the quantisation run side by side, a block takes its queue and output
+// space with one atomic per counter, and the triangles are copied by their own
+// kernel (k_emit_tris), coalesced. 655,872 triangles: 1,313 -> 194 us in eleven launches and 15 for the triangles.
+constexpr int kColBlock = 128, kColNodes = kColBlock / 8;
+__global__ void __launch_bounds__(kColBlock) k_collapse(collapse_args a) {
+  __shared__ uint32_t s_int[kColNodes], s_tri[kColNodes], s_slots[kColNodes], s_base[3];
+  __shared__ __align__(16) uint8_t s_node[kColNodes][sizeof(bvh8_node)];
+  constexpr uint32_t kAll = 0xffffffffu;
+  uint32_t const lane = threadIdx.x & 31u, sub = lane & 7u, base8 = lane & ~7u, oct = threadIdx.x >> 3;
+  uint32_t const n_in = *a.n_in;
+  for (uint32_t first = blockIdx.x * kColNodes; first < n_in; first += gridDim.x * kColNodes) {
+    uint32_t const it = first + oct;
+    bool const live = it < n_in;
+    collapse_item item{kLeafBit, 0u, 0u};
+    if (live) item = a.in[it];
+    // open the node: the child with the largest area among those of more than
+    // kMaxLeaf triangles (ties: the first) is replaced by its two children
+    uint32_t ref = kNone, cnt = 0;
+    uint2 kids = make_uint2(0u, 0u);  // ref's own children, loaded with its box
+    ibox kb{make_float4(INFINITY, INFINITY, INFINITY, 0.f), make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f)};
+    uint32_t nk = 0;
+    auto fetch = [&](uint32_t r) {
+      ref = r;
+      if (!(r & kLeafBit)) kids = a.child[r];
+      cnt = prim_count(a, r);
+      kb = load_box(r, a.leaf_boxes, a.order, a.inner);
+    };
+    if (live) {
+      if ((item.ref & kLeafBit) || prim_count(a, item.ref) <= uint32_t(kMaxLeaf)) {
+        nk = 1;  // the whole (small) tree is one leaf slot
+        if (sub == 0) fetch(item.ref);
+      } else {
+        uint2 const c = a.child[item.ref];
+        nk = 2;
+        if (sub < 2) fetch(sub == 0 ? c.x : c.y);
       }
-      if (best < 0) break;
-      uint2 const c2 = a.child[kids[best]];
-      kids[best] = c2.x;
-      kids[nk++] = c2.y;
     }
-  }
-  ibox nb = load_box(kids[0], a.leaf_boxes, a.order, a.inner);
-  kb[0] = nb;
-  for (int k = 1; k < nk; ++k) {
-    kb[k] = load_box(kids[k], a.leaf_boxes, a.order, a.inner);
-    nb = merge(nb, kb[k]);
-  }
-  float const cx = 0.5f * (nb.lo.x + nb.hi.x), cy = 0.5f * (nb.lo.y + nb.hi.y), cz = 0.5f * (nb.lo.z + nb.hi.z);
-  // octant slot assignment (the host builder's rule): slot s faces (+-1, +-1,
-  // +-1), bit a of s set meaning +; repeatedly the (child, slot) pair with the
-  // largest projection takes the slot
-  int slot_of[8];
-  {
-    bool kid_done[8] = {}, slot_done[8] = {};
-    float cost[8][8];
-    for (int k = 0; k < nk; ++k) {
-      float const dx = 0.5f * (kb[k].lo.x + kb[k].hi.x) - cx;
-      float const dy = 0.5f * (kb[k].lo.y + kb[k].hi.y) - cy;
-      float const dz = 0.5f * (kb[k].lo.z + kb[k].hi.z) - cz;
-      for (int s = 0; s < 8; ++s) cost[k][s] = ((s & 1) ? dx : -dx) + ((s & 2) ? dy : -dy) + ((s & 4) ? dz : -dz);
+#pragma unroll 1
+    for (int r = 0; r < 6; ++r) {
+      float ar = -1.f;
+      if (cnt > uint32_t(kMaxLeaf)) {
+        float const v = area(kb);
+        if (v > -1.f) ar = v;
+      }
+      uint32_t who = sub;
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) {
+        float const oa = __shfl_xor_sync(kAll, ar, o);
+        uint32_t const ow = __shfl_xor_sync(kAll, who, o);
+        if (oa > ar || (oa == ar && ow < who)) ar = oa, who = ow;
+      }
+      bool const open = ar > -1.f;
+      if (!__any_sync(kAll, open)) break;
+      uint2 const c = make_uint2(__shfl_sync(kAll, kids.x, int(base8 + who)),
+          __shfl_sync(kAll, kids.y, int(base8 + who)));
+      if (open) {
+        if (sub == who || sub == nk) fetch(sub == who ? c.x : c.y);
+        ++nk;
+      }
     }
-    for (int r = 0; r < nk; ++r) {
-      int bk = -1, bs = -1;
-      float bc = -3.402823466e38f;
-      for (int k = 0; k < nk; ++k) {
-        if (kid_done[k]) continue;
-        for (int s = 0; s < 8; ++s) {
-          if (slot_done[s]) continue;
-          if (cost[k][s] > bc) {
-            bc = cost[k][s];
-            bk = k;
-            bs = s;
+    // the node's box
+    ibox nb = kb;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      nb.lo.x = fminf(nb.lo.x, __shfl_xor_sync(kAll, nb.lo.x, o));
+      nb.lo.y = fminf(nb.lo.y, __shfl_xor_sync(kAll, nb.lo.y, o));
+      nb.lo.z = fminf(nb.lo.z, __shfl_xor_sync(kAll, nb.lo.z, o));
+      nb.hi.x = fmaxf(nb.hi.x, __shfl_xor_sync(kAll, nb.hi.x, o));
+      nb.hi.y = fmaxf(nb.hi.y, __shfl_xor_sync(kAll, nb.hi.y, o));
+      nb.hi.z = fmaxf(nb.hi.z, __shfl_xor_sync(kAll, nb.hi.z, o));
+    }
+    // octant slot assignment (the host builder's rule): slot s faces (+-1, +-1,
+    // +-1), bit a of s set meaning +; repeatedly the (child, slot) pair with the
+    // largest projection takes the slot (ties: the first child, its first slot)
+    uint32_t slot = 8u, free_slots = 0xffu;
+    {
+      float const dx = 0.5f * (kb.lo.x + kb.hi.x) - 0.5f * (nb.lo.x + nb.hi.x);
+      float const dy = 0.5f * (kb.lo.y + kb.hi.y) - 0.5f * (nb.lo.y + nb.hi.y);
+      float const dz = 0.5f * (kb.lo.z + kb.hi.z) - 0.5f * (nb.lo.z + nb.hi.z);
+      bool todo = sub < nk;
+#pragma unroll 1
+      for (uint32_t r = 0; r < 8u; ++r) {
+        float bc = -3.402823466e38f;
+        uint32_t pick = 0x800u | (sub << 4);  // 0x800: no slot above the floor (NaN boxes)
+        if (todo) {
+#pragma unroll
+          for (uint32_t s = 0; s < 8u; ++s) {
+            float const v = ((s & 1) ? dx : -dx) + ((s & 2) ? dy : -dy) + ((s & 4) ? dz : -dz);
+            if (((free_slots >> s) & 1u) && v > bc) bc = v, pick = (sub << 4) | s;
           }
+        } else {
+          pick = 0x1000u;
+        }
+        // largest projection; without one, the first child still to place
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+          float const oc = __shfl_xor_sync(kAll, bc, o);
+          uint32_t const op = __shfl_xor_sync(kAll, pick, o);
+          bool const mine = pick < 0x800u, theirs = op < 0x800u;
+          if (theirs != mine ? theirs : (theirs && oc != bc ? oc > bc : op < pick)) bc = oc, pick = op;
+        }
+        if (!__any_sync(kAll, pick < 0x1000u)) break;
+        if (pick < 0x1000u) {
+          uint32_t const s = pick < 0x800u ? pick & 15u : uint32_t(__ffs(free_slots) - 1);
+          if (((pick >> 4) & 7u) == sub) {
+            slot = s;
+            todo = false;
+          }
+          free_slots &= ~(1u << s);
         }
       }
-      if (bk < 0) {  // NaN boxes: take the first free pair
-        for (int k = 0; k < nk && bk < 0; ++k)
-          if (!kid_done[k]) bk = k;
-        for (int s = 0; s < 8 && bs < 0; ++s)
-          if (!slot_done[s]) bs = s;
-      }
-      kid_done[bk] = slot_done[bs] = true;
-      slot_of[bk] = bs;
     }
-  }
-  int slot_kid[8];
-  for (int s = 0; s < 8; ++s) slot_kid[s] = -1;
-  for (int k = 0; k < nk; ++k) slot_kid[slot_of[k]] = k;
-  uint32_t n_int = 0, n_tri = 0;
-  for (int k = 0; k < nk; ++k) {
-    uint32_t const pc = prim_count(a, kids[k]);
-    if (pc <= uint32_t(kMaxLeaf)) n_tri += pc;
-    else ++n_int;
-  }
-  uint32_t const child_base = n_int ? atomicAdd(&a.counters[0], n_int) : 0u;
-  uint32_t const tri_base = n_tri ? atomicAdd(&a.counters[1], n_tri) : 0u;
-  uint32_t const out_base = n_int ? atomicAdd(a.n_out, n_int) : 0u;
-  atomicMax(&a.counters[3], item.depth);
-
-  bvh8_node node;
-  node.px = nb.lo.x;
-  node.py = nb.lo.y;
-  node.pz = nb.lo.z;
-  node.imask = 0;
-  float const ext[3] = {nb.hi.x - nb.lo.x, nb.hi.y - nb.lo.y, nb.hi.z - nb.lo.z};
-  double scale[3];
-  for (int ax = 0; ax < 3; ++ax) {
-    node.e[ax] = biased_exponent(ext[ax]);
-    scale[ax] = ldexp(1.0, int(node.e[ax]) - 127);
-  }
-  float const p[3] = {node.px, node.py, node.pz};
-  node.child_base = child_base;
-  node.tri_base = tri_base;
-  uint32_t tri_off = 0, rank = 0, slots = 0;
-  for (int s = 0; s < 8; ++s) {
-    int const k = slot_kid[s];
-    if (k < 0) {
-      for (int ax = 0; ax < 3; ++ax) {
-        node.qlo[ax][s] = 1;
-        node.qhi[ax][s] = 0;
-      }
-      node.meta[s] = 0;
-      continue;
+    // lane = slot from here on
+    uint32_t from = 8u;
+#pragma unroll
+    for (uint32_t k = 0; k < 8u; ++k)
+      if (__shfl_sync(kAll, slot, int(base8 + k)) == sub) from = k;
+    {
+      int const src = int(base8 + (from & 7u));
+      ref = __shfl_sync(kAll, ref, src);
+      cnt = __shfl_sync(kAll, cnt, src);
+      kb.lo.x = __shfl_sync(kAll, kb.lo.x, src), kb.lo.y = __shfl_sync(kAll, kb.lo.y, src);
+      kb.lo.z = __shfl_sync(kAll, kb.lo.z, src), kb.hi.x = __shfl_sync(kAll, kb.hi.x, src);
+      kb.hi.y = __shfl_sync(kAll, kb.hi.y, src), kb.hi.z = __shfl_sync(kAll, kb.hi.z, src);
+      if (from == 8u) cnt = 0;
     }
-    float const blo[3] = {kb[k].lo.x, kb[k].lo.y, kb[k].lo.z}, bhi[3] = {kb[k].hi.x, kb[k].hi.y, kb[k].hi.z};
+    bool const internal = cnt > uint32_t(kMaxLeaf);
+    uint32_t const tris = internal ? 0u : cnt;
+    uint32_t const imask = (__ballot_sync(kAll, internal) >> base8) & 0xffu;
+    uint32_t const leaves = (__ballot_sync(kAll, tris > 0u) >> base8) & 0xffu;
+    uint32_t const rank = uint32_t(__popc(imask & ((1u << sub) - 1u)));
+    uint32_t tri_end = tris;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      uint32_t const v = __shfl_up_sync(kAll, tri_end, o, 8);
+      if (sub >= uint32_t(o)) tri_end += v;
+    }
+    uint32_t const tri_off = tri_end - tris;
+    // queue, node and triangle space of the block's nodes
+    if (sub == 7u) {
+      s_int[oct] = uint32_t(__popc(imask));
+      s_tri[oct] = tri_end;
+      s_slots[oct] = uint32_t(__popc(leaves));
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      uint32_t const i0 = lane < kColNodes ? s_int[lane] : 0u, t0 = lane < kColNodes ? s_tri[lane] : 0u;
+      uint32_t i1 = i0, t1 = t0, sl = lane < kColNodes ? s_slots[lane] : 0u;
+#pragma unroll
+      for (int o = 1; o < kColNodes; o <<= 1) {
+        uint32_t const vi = __shfl_up_sync(kAll, i1, o), vt = __shfl_up_sync(kAll, t1, o);
+        if (lane >= uint32_t(o)) i1 += vi, t1 += vt;
+      }
+      sl = __reduce_add_sync(kAll, sl);
+      if (lane < kColNodes) s_int[lane] = i1 - i0, s_tri[lane] = t1 - t0;
+      if (lane == kColNodes - 1) {
+        s_base[0] = i1 ? atomicAdd(&a.counters[0], i1) : 0u;
+        s_base[1] = t1 ? atomicAdd(&a.counters[1], t1) : 0u;
+        s_base[2] = i1 ? atomicAdd(a.n_out, i1) : 0u;
+      } else if (lane == 0) {
+        if (sl) atomicAdd(&a.counters[4], sl);
+        atomicMax(&a.counters[3], item.depth);
+      }
+    }
+    __syncthreads();
+    uint32_t const child_base = s_base[0] + s_int[oct], tri_base = s_base[1] + s_tri[oct],
+                   out_base = s_base[2] + s_int[oct];
+    // quantise the slot's box outwards
+    float const p[3] = {nb.lo.x, nb.lo.y, nb.lo.z};
+    float const ext[3] = {nb.hi.x - nb.lo.x, nb.hi.y - nb.lo.y, nb.hi.z - nb.lo.z};
+    float const blo[3] = {kb.lo.x, kb.lo.y, kb.lo.z}, bhi[3] = {kb.hi.x, kb.hi.y, kb.hi.z};
+    uint8_t* const img = s_node[oct];
+    uint32_t exps = imask << 24;
+#pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
-      double const lo = floor((double(blo[ax]) - double(p[ax])) / scale[ax]);
-      double const hi = ceil((double(bhi[ax]) - double(p[ax])) / scale[ax]);
-      node.qlo[ax][s] = uint8_t(fmin(fmax(lo, 0.0), 255.0));
-      node.qhi[ax][s] = uint8_t(fmin(fmax(hi, 0.0), 255.0));
+      uint32_t const e = biased_exponent(ext[ax]);
+      exps |= e << (8 * ax);
+      double const inv = pow2(127 - int(e));
+      double const lo = floor((double(blo[ax]) - double(p[ax])) * inv);
+      double const hi = ceil((double(bhi[ax]) - double(p[ax])) * inv);
+      img[32 + 8 * ax + sub] = cnt ? uint8_t(fmin(fmax(lo, 0.0), 255.0)) : uint8_t(1);
+      img[56 + 8 * ax + sub] = cnt ? uint8_t(fmin(fmax(hi, 0.0), 255.0)) : uint8_t(0);
     }
-    uint32_t const pc = prim_count(a, kids[k]);
-    if (pc > uint32_t(kMaxLeaf)) {
-      node.imask |= uint8_t(1u << s);
-      node.meta[s] = uint8_t(0x20u | unsigned(s));
-      a.out[out_base + rank] = collapse_item{kids[k], child_base + rank, item.depth + 1u};
-      ++rank;
-    } else {
-      node.meta[s] = uint8_t(tri_off | (pc << 5));
-      uint2 const r = prim_range(a, kids[k]);
-      for (uint32_t q = r.x; q <= r.y; ++q) {
-        uint32_t const prim = a.order[q];
-        float const* v = a.pos + 9 * size_t(prim);
-        float4* t = a.tris + 3 * size_t(tri_base + tri_off);
-        t[0] = make_float4(v[0], v[1], v[2], __uint_as_float(prim));
-        t[1] = make_float4(v[3], v[4], v[5], 0.f);
-        t[2] = make_float4(v[6], v[7], v[8], 0.f);
-        ++tri_off;
+    img[24 + sub] = internal ? uint8_t(0x20u | sub) : (cnt ? uint8_t(tri_off | (cnt << 5)) : uint8_t(0));
+    if (sub == 0) {
+      uint32_t* const h = reinterpret_cast<uint32_t*>(img);
+      h[0] = __float_as_uint(p[0]), h[1] = __float_as_uint(p[1]), h[2] = __float_as_uint(p[2]);
+      h[3] = exps;
+      h[4] = __popc(imask) ? child_base : 0u;
+      h[5] = leaves ? tri_base : 0u;
+    }
+    __syncwarp();
+    if (live) {
+      if (sub < 5u) reinterpret_cast<uint4*>(a.nodes + item.wide)[sub] = reinterpret_cast<uint4 const*>(img)[sub];
+      if (internal) {
+        a.out[out_base + rank] = collapse_item{ref, child_base + rank, item.depth + 1u};
+      } else if (cnt) {
+        uint32_t const q = (ref & kLeafBit) ? (ref & ~kLeafBit) : a.range[ref].x;
+        for (uint32_t i = 0; i < cnt; ++i) a.tri_prim[tri_base + tri_off + i] = a.order[q + i];
       }
-      ++slots;
     }
+    __syncthreads();  // the shared arrays are reused
   }
-  if (slots) atomicAdd(&a.counters[4], slots);
-  a.nodes[item.wide] = node;
+}
+
+// Leaf-ordered triangles from their prims.
+__global__ void k_emit_tris(float const* __restrict__ pos, uint32_t const* __restrict__ tri_prim, uint32_t n,
+    float4* __restrict__ tris) {
+  uint32_t const t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  uint32_t const prim = tri_prim[t];
+  float const* v = pos + 9 * size_t(prim);
+  float4* o = tris + 3 * size_t(t);
+  o[0] = make_float4(v[0], v[1], v[2], __uint_as_float(prim));
+  o[1] = make_float4(v[3], v[4], v[5], 0.f);
+  o[2] = make_float4(v[6], v[7], v[8], 0.f);
 }
 
 template <typename T> int dalloc(T** p, size_t count, std::vector<void*>& owned) {
@@ -414,8 +540,8 @@ int build_bvh8_device(float const* d_pos, size_t n_tris, cudaStream_t st, device
   carve c;
   size_t const o_boxes = c.take<ibox>(n), o_cb = c.take<uint32_t>(6), o_k0 = c.take<uint64_t>(n),
                o_k1 = c.take<uint64_t>(n), o_v0 = c.take<uint32_t>(n), o_v1 = c.take<uint32_t>(n),
-               o_child = c.take<uint2>(n), o_range = c.take<uint2>(n), o_par_i = c.take<uint32_t>(n),
-               o_par_l = c.take<uint32_t>(n), o_arrivals = c.take<uint32_t>(n), o_counters = c.take<uint32_t>(8),
+               o_child = c.take<uint2>(n), o_range = c.take<uint2>(n), o_cross = c.take<uint32_t>(n),
+               o_blocks = c.take<ibox>(size_t(n) / kBoxBlock + 1), o_counters = c.take<uint32_t>(8 + kMaxLevels + 1),
                o_inner = c.take<ibox>(n), o_q0 = c.take<collapse_item>(n), o_q1 = c.take<collapse_item>(n),
                o_temp = c.take<char>(tb);
   if (scratch.bytes < c.total) {
@@ -436,9 +562,8 @@ int build_bvh8_device(float const* d_pos, size_t n_tris, cudaStream_t st, device
   auto* const v1 = reinterpret_cast<uint32_t*>(B + o_v1);
   auto* const child = reinterpret_cast<uint2*>(B + o_child);
   auto* const range = reinterpret_cast<uint2*>(B + o_range);
-  auto* const par_i = reinterpret_cast<uint32_t*>(B + o_par_i);
-  auto* const par_l = reinterpret_cast<uint32_t*>(B + o_par_l);
-  auto* const arrivals = reinterpret_cast<uint32_t*>(B + o_arrivals);
+  auto* const cross = reinterpret_cast<uint32_t*>(B + o_cross);
+  auto* const block_box = reinterpret_cast<ibox*>(B + o_blocks);
   auto* const counters = reinterpret_cast<uint32_t*>(B + o_counters);
   auto* const inner = reinterpret_cast<ibox*>(B + o_inner);
   collapse_item* const q[2] = {reinterpret_cast<collapse_item*>(B + o_q0), reinterpret_cast<collapse_item*>(B + o_q1)};
@@ -468,24 +593,25 @@ int build_bvh8_device(float const* d_pos, size_t n_tris, cudaStream_t st, device
     *what = w;
     return err;
   };
-  // counters: [0] wide nodes (the root), [2] level-0 queue length (the root item)
+  // counters: [0] wide nodes (the root); lens[l]: level l's queue length (level 0: the root item)
   static uint32_t const init_cb[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
-  static uint32_t const init_counters[8] = {1u, 0u, 1u, 0u, 0u, 0u, 0u, 0u};
+  static uint32_t const init_counters[9] = {1u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 1u};
+  uint32_t* const lens = counters + 8;
   collapse_item const root{n >= 2 ? 0u : kLeafBit, 0u, 1u};
   cudaMemcpyAsync(cb, init_cb, sizeof init_cb, cudaMemcpyHostToDevice, st);
+  cudaMemsetAsync(counters, 0, (8 + kMaxLevels + 1) * sizeof(uint32_t), st);
   cudaMemcpyAsync(counters, init_counters, sizeof init_counters, cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(q[0], &root, sizeof root, cudaMemcpyHostToDevice, st);
-  cudaMemsetAsync(par_i, 0xff, size_t(n) * 4, st);
-  cudaMemsetAsync(par_l, 0xff, size_t(n) * 4, st);
-  cudaMemsetAsync(arrivals, 0, size_t(n) * 4, st);
   uint32_t const blocks = uint32_t((n + 255) / 256);
   k_prim_boxes<<<blocks, 256, 0, st>>>(d_pos, uint32_t(n), 1e-5f, boxes, cb);
   k_morton<<<blocks, 256, 0, st>>>(boxes, uint32_t(n), cb, k0, v0);
   if ((e = int(cub::DeviceRadixSort::SortPairs(temp, tb, k0, k1, v0, v1, n, 0, 63, st))))
     return fail(e, "device BVH sort");
   if (n >= 2) {
-    k_radix_tree<<<uint32_t((n - 1 + 255) / 256), 256, 0, st>>>(k1, n, child, range, par_i, par_l);
-    k_boxes_up<<<blocks, 256, 0, st>>>(boxes, v1, n, child, par_i, par_l, arrivals, inner);
+    k_radix_tree<<<uint32_t((n - 1 + 255) / 256), 256, 0, st>>>(k1, n, child, range);
+    k_boxes_block<<<uint32_t((n + kBoxBlock - 1) / kBoxBlock), kBoxBlock, 0, st>>>(boxes, v1, n, range, inner,
+        block_box, cross, counters + 2);
+    k_boxes_cross<<<kCrossGrid, 256, 0, st>>>(boxes, v1, range, block_box, cross, counters + 2, inner);
   }
   collapse_args ca{};
   ca.leaf_boxes = boxes;
@@ -493,34 +619,36 @@ int build_bvh8_device(float const* d_pos, size_t n_tris, cudaStream_t st, device
   ca.child = child;
   ca.range = range;
   ca.inner = inner;
-  ca.pos = d_pos;
   ca.nodes = nodes;
-  ca.tris = tris;
+  ca.tri_prim = v0;  // the sort's input order, no longer needed
   ca.counters = counters;
-  ca.n = n;
-  // Level l reads queue l & 1 (length in counters[2] or [5]) and appends to
-  // the other. Levels are launched in batches without reading their lengths
-  // back: a level holds at most 8^l items (and at most n), which sizes its
-  // grid; threads past the device-side length return at once. One read-back
-  // per batch finds the end.
-  uint32_t hc[8];
+  // Level l reads queue l & 1, lens[l] items long, and appends to the other.
+  // Levels are launched in batches without reading their lengths back: a
+  // level holds at most 8^l items (and at most n), which sizes its grid, up to
+  // a fixed number of blocks that then loop. The first batch is what a tree of
+  // n triangles usually has (an eighth per level down to 2 triangles, and 4
+  // more); one read-back per batch finds the end.
+  uint32_t hc[8], len = 1;
   uint32_t bound = 1;
-  for (int level = 0;;) {
-    for (int b = 0; b < 8; ++b, ++level) {
+  int batch = 4;
+  for (size_t m = n_tris / 2; m > 0; m /= 8) ++batch;
+  for (int level = 0; len;) {
+    if (level + batch > kMaxLevels) return fail(-1, "device BVH collapse did not finish");
+    for (int b = 0; b < batch; ++b, ++level) {
       int const in = level & 1;
-      uint32_t* const len_out = counters + (in ? 2 : 5);
-      cudaMemsetAsync(len_out, 0, 4, st);
       ca.in = q[in];
-      ca.n_in = counters + (in ? 5 : 2);
+      ca.n_in = lens + level;
       ca.out = q[in ^ 1];
-      ca.n_out = len_out;
-      k_collapse<<<(bound + 127) / 128, 128, 0, st>>>(ca);
+      ca.n_out = lens + level + 1;
+      k_collapse<<<std::min<uint32_t>((bound + kColNodes - 1) / kColNodes, kColGrid), kColBlock, 0, st>>>(ca);
       bound = uint32_t(std::min<uint64_t>(uint64_t(bound) * 8u, uint64_t(n)));
     }
+    // complete once no level is left; until then v0 holds valid prims
+    k_emit_tris<<<blocks, 256, 0, st>>>(d_pos, v0, uint32_t(n), tris);
     cudaMemcpyAsync(hc, counters, sizeof hc, cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(&len, lens + level, sizeof len, cudaMemcpyDeviceToHost, st);
     if ((e = int(cudaStreamSynchronize(st)))) return fail(e, "device BVH collapse");
-    if (hc[(level & 1) ? 5 : 2] == 0) break;  // the next level's queue is empty
-    if (level > 4096) return fail(-1, "device BVH collapse did not finish");
+    batch = 4;
   }
   if ((e = int(cudaGetLastError()))) return fail(e, "device BVH launch");
   out.nodes = nodes;
