@@ -68,6 +68,8 @@ struct guide_state {
   size_t records_cap = 0;        // in records
   float4* samples = nullptr;     // 4 float4 per sample
   size_t samples_cap = 0;
+  void* call_buf = nullptr;      // inputs and outputs of the host-array calls (call_buffer)
+  size_t call_cap = 0;
   myrt_guide_params prm{0.5f, 1e-2f, 16u, 16384u, 1u, 1u, 1u, 10.f, 0u, 0u};
   uint32_t wave = 0;
   uint32_t tag = 0;
@@ -89,75 +91,8 @@ struct mlp_args {
                         // (exercises the timeout path; the MMA in flight is still drained)
 };
 
-// ---- encoding ------------------------------------------------------------------------
-__device__ __forceinline__ void encode(mlp_args const& a, float4 p, float4 n, float4 wo, float (&f)[64]) {
-  float pn[3] = {(p.x - a.center[0]) * a.inv_half[0], (p.y - a.center[1]) * a.inv_half[1],
-      (p.z - a.center[2]) * a.inv_half[2]};
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    pn[k] = fminf(fmaxf(pn[k], -1.f), 1.f);
-    f[k] = pn[k];
-  }
-  // sin / cos of 2^f pi p: one sincospi per axis, then the double-angle
-  // formulas (the features are rounded to BF16 before the first layer, far
-  // above the recurrence's few-ulp drift)
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    float s, c;
-    sincospif(pn[k], &s, &c);
-#pragma unroll
-    for (int fr = 0; fr < 6; ++fr) {
-      f[3 + 6 * fr + 2 * k] = s;
-      f[4 + 6 * fr + 2 * k] = c;
-      float const s2 = 2.f * s * c;
-      c = fmaf(-2.f * s, s, 1.f);
-      s = s2;
-    }
-  }
-  f[39] = n.x, f[40] = n.y, f[41] = n.z;
-  f[42] = wo.x, f[43] = wo.y, f[44] = wo.z;
-  f[45] = 1.f;
-#pragma unroll
-  for (int k = 46; k < 64; ++k) f[k] = 0.f;
-}
-
-// 64 floats -> one swizzled BF16 row of a tile
-__device__ __forceinline__ void store_row(uint8_t* tile, uint32_t r, float const (&f)[64]) {
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    uint4 v;
-    v.x = tc::pack_bf16(f[8 * c + 0], f[8 * c + 1]);
-    v.y = tc::pack_bf16(f[8 * c + 2], f[8 * c + 3]);
-    v.z = tc::pack_bf16(f[8 * c + 4], f[8 * c + 5]);
-    v.w = tc::pack_bf16(f[8 * c + 6], f[8 * c + 7]);
-    *reinterpret_cast<uint4*>(tile + tc::sw128_offset(r, uint32_t(c))) = v;
-  }
-}
 __device__ __forceinline__ float bf16_lo(uint32_t u) { return __uint_as_float(u << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
-__device__ __forceinline__ void load_row(uint8_t const* tile, uint32_t r, float (&f)[64]) {
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    uint4 const v = *reinterpret_cast<uint4 const*>(tile + tc::sw128_offset(r, uint32_t(c)));
-    f[8 * c + 0] = bf16_lo(v.x), f[8 * c + 1] = bf16_hi(v.x);
-    f[8 * c + 2] = bf16_lo(v.y), f[8 * c + 3] = bf16_hi(v.y);
-    f[8 * c + 4] = bf16_lo(v.z), f[8 * c + 5] = bf16_hi(v.z);
-    f[8 * c + 6] = bf16_lo(v.w), f[8 * c + 7] = bf16_hi(v.w);
-  }
-}
-
-// the accumulator row of this thread (64 columns starting at col) + bias
-__device__ __forceinline__ void acc_row(uint32_t tmem, uint32_t col, float const* bias, float (&f)[64]) {
-  uint32_t const warp = threadIdx.x >> 5;
-  float lo[32], hi[32];
-  tc::tmem_ld32(tmem + ((32u * warp) << 16) + col, lo);
-  tc::tmem_ld32(tmem + ((32u * warp) << 16) + col + 32u, hi);
-#pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    f[j] = lo[j] + (bias ? bias[j] : 0.f);
-    f[32 + j] = hi[j] + (bias ? bias[32 + j] : 0.f);
-  }
-}
 
 // weights (bf16 [4][64][64]) -> four swizzled 64 x 64 tiles; biases -> smem
 __device__ __forceinline__ void load_weights(mlp_args const& a, uint8_t* wt, float* bias) {
@@ -170,45 +105,7 @@ __device__ __forceinline__ void load_weights(mlp_args const& a, uint8_t* wt, flo
 }
 
 // ---- mixture parameters -----------------------------------------------------------------
-struct lobe_set {
-  float w[kGuideLobes], kappa[kGuideLobes], mu[kGuideLobes][3], len[kGuideLobes], dk[kGuideLobes];
-};
 constexpr float kKappaMin = 0.01f, kKappaMax = 1000.f;
-
-__device__ __forceinline__ void mixture(float const (&o)[64], lobe_set& L) {
-  float mx = o[0];
-#pragma unroll
-  for (int k = 1; k < kGuideLobes; ++k) mx = fmaxf(mx, o[5 * k]);
-  float sum = 0.f;
-#pragma unroll
-  for (int k = 0; k < kGuideLobes; ++k) {
-    L.w[k] = __expf(o[5 * k] - mx);
-    sum += L.w[k];
-  }
-#pragma unroll
-  for (int k = 0; k < kGuideLobes; ++k) {
-    L.w[k] = L.w[k] / sum;
-    float const x = o[5 * k + 1];
-    float const ex = __expf(-fabsf(x));  // softplus(x) = max(x, 0) + log(1 + e^-|x|)
-    float const sp = fmaxf(x, 0.f) + log1pf(ex);
-    float kap = sp + kKappaMin;
-    float dk = x >= 0.f ? __frcp_rn(1.f + ex) : ex * __frcp_rn(1.f + ex);  // d softplus / dx
-    if (kap > kKappaMax) {
-      kap = kKappaMax;
-      dk = 0.f;
-    }
-    L.kappa[k] = kap;
-    L.dk[k] = dk;
-    float const mx3 = o[5 * k + 2], my = o[5 * k + 3], mz = o[5 * k + 4];
-    float const len = sqrtf(mx3 * mx3 + my * my + mz * mz);
-    L.len[k] = len;
-    if (len > 1e-6f) {
-      L.mu[k][0] = mx3 / len, L.mu[k][1] = my / len, L.mu[k][2] = mz / len;
-    } else {
-      L.mu[k][0] = 0.f, L.mu[k][1] = 0.f, L.mu[k][2] = 1.f;
-    }
-  }
-}
 // kappa / (2 pi (1 - exp(-2 kappa)))
 __device__ __forceinline__ float vmf_norm(float k) { return k / (-6.28318530717958648f * expm1f(-2.f * k)); }
 
@@ -251,10 +148,14 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
   return p + ((1024u - (s & 1023u)) & 1023u);
 }
 
-// Encoding of one point (as encode()) written to row r of a swizzled tile in
-// eight 16-byte chunks, each stored as soon as its 8 features exist.
+// Encoding of one point written to row r of a swizzled tile in eight 16-byte
+// chunks, each stored as soon as its 8 features exist (chunks first .. last of
+// them; the caller's threads of one row may share them out). sin / cos of
+// 2^f pi p: one sincospi per axis, then the double-angle formulas (the features
+// are rounded to BF16 before the first layer, far above the recurrence's
+// few-ulp drift).
 __device__ __forceinline__ void encode_store(mlp_args const& a, float4 p, float4 n, float4 wo, uint8_t* tile,
-    uint32_t r) {
+    uint32_t r, uint32_t first = 0, uint32_t last = 7) {
   float pn[3] = {(p.x - a.center[0]) * a.inv_half[0], (p.y - a.center[1]) * a.inv_half[1],
       (p.z - a.center[2]) * a.inv_half[2]};
   float sn[3], cs[3];
@@ -266,7 +167,7 @@ __device__ __forceinline__ void encode_store(mlp_args const& a, float4 p, float4
   float buf[8];
   auto put = [&](int i, float v) {
     buf[i & 7] = v;
-    if ((i & 7) == 7) {
+    if ((i & 7) == 7 && uint32_t(i >> 3) >= first && uint32_t(i >> 3) <= last) {
       uint4 q;
       q.x = tc::pack_bf16(buf[0], buf[1]);
       q.y = tc::pack_bf16(buf[2], buf[3]);
@@ -322,7 +223,7 @@ __device__ __forceinline__ void relu_to_tile(uint32_t tacc, float const* bias, u
   }
 }
 
-// Output layer of one row -> its mixture (as mixture()) as 16 float4:
+// Output layer of one row -> its mixture as 16 float4:
 // o[k] = (mu, kappa), o[8 + k] = (w, vmf normaliser, cdf, flag on k = 0).
 // The first eight go to row r of the swizzled staging tile `st` (the group's H
 // tile, free once the last layer's MMA is done), the other eight to the row's
@@ -540,12 +441,31 @@ __global__ void __launch_bounds__(256) k_guide_collect(float4 const* __restrict_
 }
 
 // ---- k_guide_train -----------------------------------------------------------------------------
-// Shared memory: W 4 x 8 KB | H0..H3 4 x 16 KB | dZ 16 KB | zero 16 KB | bias 1 KB |
-// dbias 1 KB | per-row (wi, weight) 2 KB | mbarrier | TMEM address | stall-test mbarrier.
-constexpr uint32_t kTrW = 0, kTrH = 32768, kTrDZ = 98304, kTrZero = 114688, kTrBias = 131072, kTrDBias = 132096,
-                   kTrRow = 133120, kTrBar = 135168, kTrTmem = 135176, kTrStall = 135184;
-constexpr uint32_t kTrSmem = 135192 + 1024;
+// A batch of 16,384 samples is one 128-row tile for most SMs, so a step is the
+// latency of one tile: 8 dependent tensor-core passes with the row work between
+// them. Sixteen warps share a tile: warp w owns rows 32 (w % 4) .. + 31 (its TMEM
+// lanes) and part w / 4 of their columns -- 16 of a layer's 64, two of the eight
+// lobes -- so four warps a scheduler cover one another's waits and every row's
+// loss is computed by four threads (which exchange exponentials and lobe
+// densities through shared memory and sum them in lobe order). Bias gradients
+// are column sums over a warp's rows by recursive halving (16 shuffles for 16
+// columns instead of 80, the additions those of a full butterfly), added up in
+// a fixed order; the data gradient's MMAs are committed before the weight
+// gradients', which then run under the next layer's row work, with dZ in two
+// buffers. One thread per row, a butterfly and a shared atomic per column and
+// one dZ buffer took 62 us per 16,384-sample step; this takes 20 us (ncu).
+//
+// Shared memory: W 4 x 8 KB | H0..H3 4 x 16 KB | dZ 2 x 16 KB | zero 16 KB | bias 1 KB | dbias 1 KB |
+// per-row (wi, weight) 2 KB | per-row exchange 128 x 24 floats | bias sums of a tile, by layer, quarter and
+// column 4 KB | mbarrier | TMEM address | stall-test mbarrier.
+constexpr uint32_t kTrParts = 4, kTrThreads = 128 * kTrParts;
+constexpr uint32_t kTrW = 0, kTrH = 32768, kTrDZ = 98304, kTrZero = 131072, kTrBias = 147456, kTrDBias = 148480,
+                   kTrRow = 149504, kTrEx = 151552, kTrPart = 163840, kTrBar = 167936, kTrTmem = 167944,
+                   kTrStall = 167952;
+constexpr uint32_t kTrSmem = 167960 + 1024;
+constexpr uint32_t kExStride = 24;   // floats per row: 8 logits, 8 exponentials, 8 densities
 constexpr uint32_t kTmemCols = 512;  // accumulator (64) + dW for 4 layers (4 x 64)
+constexpr uint32_t kTmemDW = 64;
 
 struct train_args {
   mlp_args m;
@@ -561,30 +481,39 @@ struct train_args {
   float* loss;            // loss sum (atomic)
 };
 
-__device__ __forceinline__ void warp_bias_sum(float const (&g)[64], float* dst) {
+// Sums v[c] over the warp's lanes; lane i gets column i / 2's. The additions are
+// those of a butterfly over lane distances 16, 8, 4, 2, 1.
+__device__ __forceinline__ float warp_column_sum(float (&v)[16]) {
+  uint32_t const lane = threadIdx.x & 31u;
 #pragma unroll
-  for (int j = 0; j < 64; ++j) {
-    float v = g[j];
+  for (int h = 8; h >= 1; h >>= 1) {
+    bool const upper = lane & uint32_t(2 * h);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(dst + j, v);
+    for (int c = 0; c < h; ++c) {
+      float const send = upper ? v[c] : v[c + h], keep = upper ? v[c + h] : v[c];
+      v[c] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * h);
+    }
   }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-__global__ void __launch_bounds__(128, 1) k_guide_train(train_args a) {
+__global__ void __launch_bounds__(kTrThreads, 1) k_guide_train(train_args a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = align1024(smem_raw);
   uint8_t* wt = sm + kTrW;
-  uint8_t* dz = sm + kTrDZ;
-  uint8_t* zt = sm + kTrZero;
   float* bias = reinterpret_cast<float*>(sm + kTrBias);
   float* dbias = reinterpret_cast<float*>(sm + kTrDBias);
   float4* rowd = reinterpret_cast<float4*>(sm + kTrRow);
+  float* bias_part = reinterpret_cast<float*>(sm + kTrPart);  // [layer][quarter][64]
   uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kTrBar);
   uint64_t* stall_bar = reinterpret_cast<uint64_t*>(sm + kTrStall);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + kTrTmem);
   uint32_t const tid = threadIdx.x, warp = tid >> 5;
+  uint32_t const quarter = warp & 3u, part = warp >> 2;  // TMEM lanes; columns 16 part .. + 15, lobes 2 part, + 1
+  uint32_t const trow = 32u * quarter + (tid & 31u);     // row of the tile
+  float* const ex = reinterpret_cast<float*>(sm + kTrEx) + kExStride * trow;
   auto H = [&](int l) { return sm + kTrH + uint32_t(l) * 16384u; };
+  auto DZ = [&](int l) { return sm + kTrDZ + uint32_t(l & 1) * 16384u; };
 
   if (warp == 0) {
     tc::tmem_alloc(tmem_slot, kTmemCols);
@@ -595,13 +524,16 @@ __global__ void __launch_bounds__(128, 1) k_guide_train(train_args a) {
     tc::mbar_init(stall_bar, 1);
   }
   load_weights(a.m, wt, bias);
-  for (uint32_t i = tid; i < 16384 / 16; i += blockDim.x) reinterpret_cast<uint4*>(zt)[i] = make_uint4(0, 0, 0, 0);
+  for (uint32_t i = tid; i < 16384 / 16; i += blockDim.x)
+    reinterpret_cast<uint4*>(sm + kTrZero)[i] = make_uint4(0, 0, 0, 0);
   for (uint32_t i = tid; i < kLayers * 64; i += blockDim.x) dbias[i] = 0.f;
+  for (uint32_t i = tid; i < kLayers * 4 * 64; i += blockDim.x) bias_part[i] = 0.f;  // columns 40 .. 63 of layer 3 stay so
   tc::fence_proxy_async();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   uint32_t const tmem = *tmem_slot;
+  uint32_t const tacc = tmem + ((32u * quarter) << 16) + 16u * part;  // this thread's accumulator columns
 
   uint32_t const avail = a.count ? min(*a.count, a.capacity) : a.n_fixed;
   uint32_t n = min(avail, a.batch);
@@ -637,19 +569,39 @@ __global__ void __launch_bounds__(128, 1) k_guide_train(train_args a) {
     tc::fence_after_sync();
     return !bad;
   };
+  // column sums over this warp's rows of BF16 pairs v (this thread's columns c0 .. c0 + 2 n - 1)
+  auto bias_sums = [&](int l, uint32_t c0, uint32_t const* v, int n) {
+    float f[16];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      f[2 * j] = j < n ? bf16_lo(v[j]) : 0.f;
+      f[2 * j + 1] = j < n ? bf16_hi(v[j]) : 0.f;
+    }
+    float const sum = warp_column_sum(f);
+    uint32_t const c = (tid & 31u) >> 1;
+    if (!(tid & 1u) && c < uint32_t(2 * n)) bias_part[(uint32_t(l) * 4u + quarter) * 64u + c0 + c] = sum;
+  };
+  // 16 values of this thread's columns -> their two BF16 chunks of a tile's row
+  auto store16 = [&](uint8_t* tile, uint32_t const (&v)[8]) {
+    *reinterpret_cast<uint4*>(tile + tc::sw128_offset(trow, 2u * part)) = make_uint4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<uint4*>(tile + tc::sw128_offset(trow, 2u * part + 1u)) = make_uint4(v[4], v[5], v[6], v[7]);
+  };
 
   for (uint32_t tile = blockIdx.x; tile * 128u < n && !failed; tile += gridDim.x) {
-    uint32_t const row = tile * 128u + tid;
+    uint32_t const row = tile * 128u + trow;
     bool const valid = row < n;
-    float f[64];
-    float4 s0{0.f, 0.f, 0.f, 0.f}, s1{0.f, 0.f, 1.f, 0.f}, s2{0.f, 0.f, 1.f, 0.f}, s3{0.f, 0.f, 1.f, 0.f};
+    float4 s0{0.f, 0.f, 0.f, 0.f}, s1{0.f, 0.f, 1.f, 0.f}, s2{0.f, 0.f, 1.f, 0.f};
     if (valid) {
       float4 const* s = a.samples + size_t(first + row) * 4;
-      s0 = s[0], s1 = s[1], s2 = s[2], s3 = s[3];
+      s0 = s[0], s1 = s[1], s2 = s[2];
+      if (part == 3u) {
+        float4 const s3 = s[3];
+        rowd[trow] = make_float4(s3.x, s3.y, s3.z, fminf(s0.w * scale, wmax));
+      }
+    } else if (part == 3u) {
+      rowd[trow] = make_float4(0.f, 0.f, 1.f, 0.f);
     }
-    rowd[tid] = make_float4(s3.x, s3.y, s3.z, valid ? fminf(s0.w * scale, wmax) : 0.f);
-    encode(a.m, s0, s1, s2, f);
-    store_row(H(0), tid, f);
+    encode_store(a.m, s0, s1, s2, H(0), trow, 2u * part, 2u * part + 1u);
     // forward
     for (int l = 0; l < kLayers && !failed; ++l) {
       sync_for_mma();
@@ -666,117 +618,186 @@ __global__ void __launch_bounds__(128, 1) k_guide_train(train_args a) {
         failed = true;
         break;
       }
-      acc_row(tmem, 0, bias + 64 * l, f);
       if (l < kLayers - 1) {
+        float v[16];
+        tc::tmem_ld16(tacc, v);
+        float const* b = bias + 64 * l + 16u * part;
+        uint32_t q[8];
 #pragma unroll
-        for (int j = 0; j < 64; ++j) f[j] = fmaxf(f[j], 0.f);
-        store_row(H(l + 1), tid, f);
+        for (int j = 0; j < 8; ++j) q[j] = tc::pack_bf16_relu(v[2 * j] + b[2 * j], v[2 * j + 1] + b[2 * j + 1]);
+        store16(H(l + 1), q);
       }
     }
     if (failed) break;
-    // loss gradient w.r.t. the 40 outputs
+    // loss gradient w.r.t. the 40 outputs: this thread's lobes 2 part and 2 part + 1
     {
-      float4 const rd = rowd[tid];
+      float4 const rd = rowd[trow];
       float const wgt = rd.w;
-      lobe_set L;
-      mixture(f, L);
-      float fk[kGuideLobes], ck[kGuideLobes];
-      float q = 0.f;
+      float o[10];  // columns 10 part .. 10 part + 9, of the 16 that start at 8 part
+      {
+        float v[16];
+        tc::tmem_ld16(tmem + ((32u * quarter) << 16) + 8u * part, v);
+        float const* b = bias + 64 * 3 + 10u * part;
 #pragma unroll
-      for (int k = 0; k < kGuideLobes; ++k) {
-        ck[k] = (L.mu[k][0] * rd.x + L.mu[k][1] * rd.y) + L.mu[k][2] * rd.z;
-        fk[k] = vmf_norm(L.kappa[k]) * expf(L.kappa[k] * (ck[k] - 1.f));
-        q += L.w[k] * fk[k];
+        for (int j = 0; j < 10; ++j)
+          o[j] = (part == 0 ? v[j] : part == 1 ? v[j + 2] : part == 2 ? v[j + 4] : v[j + 6]) + b[j];
       }
-      float g[64];
+      ex[2u * part] = o[0];
+      ex[2u * part + 1u] = o[5];
+      tc::named_bar_sync(1u + quarter, 128);  // the four warps of these rows
+      float mx = ex[0];
 #pragma unroll
-      for (int j = 0; j < 64; ++j) g[j] = 0.f;
+      for (int k = 1; k < kGuideLobes; ++k) mx = fmaxf(mx, ex[k]);
+      // The roundings are written out (which products fuse into an addition):
+      // a rounding elsewhere moves some of the BF16 output gradients, and over
+      // a few Adam steps that grows to 1e-3 of the parameters.
+      float kappa[2], mu[2][3], len[2], dk[2], ck[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        float const x = o[5 * i + 1];
+        float const e1 = __expf(-fabsf(x));  // softplus(x) = max(x, 0) + log(1 + e^-|x|)
+        float kap = __fadd_rn(__fadd_rn(fmaxf(x, 0.f), log1pf(e1)), kKappaMin);
+        float d = __frcp_rn(__fadd_rn(1.f, e1));  // d softplus / dx
+        if (!(x >= 0.f)) d = __fmul_rn(e1, d);
+        if (kap > kKappaMax) {
+          kap = kKappaMax;
+          d = 0.f;
+        }
+        kappa[i] = kap;
+        dk[i] = d;
+        float const mx3 = o[5 * i + 2], my = o[5 * i + 3], mz = o[5 * i + 4];
+        float const ln = __fsqrt_rn(__fmaf_rn(mz, mz, __fmaf_rn(mx3, mx3, __fmul_rn(my, my))));
+        len[i] = ln;
+        if (ln > 1e-6f) {
+          mu[i][0] = __fdiv_rn(mx3, ln), mu[i][1] = __fdiv_rn(my, ln), mu[i][2] = __fdiv_rn(mz, ln);
+        } else {
+          mu[i][0] = 0.f, mu[i][1] = 0.f, mu[i][2] = 1.f;
+        }
+        ck[i] = __fmaf_rn(mu[i][2], rd.z, __fmaf_rn(mu[i][0], rd.x, __fmul_rn(mu[i][1], rd.y)));
+        ex[8u + 2u * part + uint32_t(i)] = __expf(__fsub_rn(o[5 * i], mx));
+        ex[16u + 2u * part + uint32_t(i)] = __fmul_rn(vmf_norm(kap), expf(__fmul_rn(kap, __fsub_rn(ck[i], 1.f))));
+      }
+      tc::named_bar_sync(1u + quarter, 128);
+      float sum = 0.f, q = 0.f;
+#pragma unroll
+      for (int k = 0; k < kGuideLobes; ++k) sum = __fadd_rn(sum, ex[8 + k]);
+#pragma unroll
+      for (int k = 0; k < kGuideLobes; ++k) q = __fadd_rn(q, __fmul_rn(__fdiv_rn(ex[8 + k], sum), ex[16 + k]));
+      float g[10];
+#pragma unroll
+      for (int j = 0; j < 10; ++j) g[j] = 0.f;
       if (wgt > 0.f && q > 1e-30f) {
-        loss_acc += -wgt * logf(q);
-        float const gq = -wgt / q;  // d loss / d q
+        if (part == 0u) loss_acc += -wgt * logf(q);
+        float const gq = __fdiv_rn(-wgt, q);  // d loss / d q
 #pragma unroll
-        for (int k = 0; k < kGuideLobes; ++k) {
-          float const kap = L.kappa[k];
-          float const wf = L.w[k] * fk[k];
-          g[5 * k] = gq * L.w[k] * (fk[k] - q);
-          float const dlnc = 1.f / kap - 2.f / expm1f(2.f * kap);
-          g[5 * k + 1] = gq * wf * (dlnc + (ck[k] - 1.f)) * L.dk[k];
-          if (L.len[k] > 1e-6f) {
-            float const gm = gq * wf * kap;  // d loss / d (mu . wi)
-            float const dmu[3] = {gm * rd.x, gm * rd.y, gm * rd.z};
-            float const proj = (dmu[0] * L.mu[k][0] + dmu[1] * L.mu[k][1]) + dmu[2] * L.mu[k][2];
+        for (int i = 0; i < 2; ++i) {
+          float const kap = kappa[i];
+          float const w = __fdiv_rn(ex[8u + 2u * part + uint32_t(i)], sum), fk = ex[16u + 2u * part + uint32_t(i)];
+          float const gwf = __fmul_rn(gq, __fmul_rn(w, fk));
+          g[5 * i] = __fmul_rn(__fmul_rn(gq, w), __fsub_rn(fk, q));
+          float const dlnc = __fsub_rn(__fdiv_rn(1.f, kap), __fdiv_rn(2.f, expm1f(__fmul_rn(2.f, kap))));
+          g[5 * i + 1] = __fmul_rn(__fmul_rn(gwf, __fadd_rn(dlnc, __fsub_rn(ck[i], 1.f))), dk[i]);
+          if (len[i] > 1e-6f) {
+            float const gm = __fmul_rn(gwf, kap);  // d loss / d (mu . wi)
+            float const dmu[3] = {__fmul_rn(gm, rd.x), __fmul_rn(gm, rd.y), __fmul_rn(gm, rd.z)};
+            float const proj =
+                __fmaf_rn(dmu[2], mu[i][2], __fmaf_rn(dmu[0], mu[i][0], __fmul_rn(dmu[1], mu[i][1])));
 #pragma unroll
-            for (int c = 0; c < 3; ++c) g[5 * k + 2 + c] = (dmu[c] - proj * L.mu[k][c]) / L.len[k];
+            for (int c = 0; c < 3; ++c) g[5 * i + 2 + c] = __fdiv_rn(__fmaf_rn(-proj, mu[i][c], dmu[c]), len[i]);
           }
         }
       }
-      store_row(dz, tid, g);
-      // bias gradient of the output layer from the BF16 values the MMAs see
-      load_row(dz, tid, g);
-      warp_bias_sum(g, dbias + 64 * 3);
+      uint8_t* const dz = DZ(kLayers - 1);
+      uint32_t gp[8];
+#pragma unroll
+      for (uint32_t j = 0; j < 5u; ++j) {  // column pairs 10 part + 2 j, + 1
+        uint32_t const c = 10u * part + 2u * j;
+        gp[j] = tc::pack_bf16(g[2 * j], g[2 * j + 1]);
+        *reinterpret_cast<uint32_t*>(dz + tc::sw128_offset(trow, c >> 3) + 2u * (c & 7u)) = gp[j];
+      }
+      if (part < 3u)  // the unused columns 40 .. 63
+        *reinterpret_cast<uint4*>(dz + tc::sw128_offset(trow, 5u + part)) = make_uint4(0, 0, 0, 0);
+      bias_sums(kLayers - 1, 10u * part, gp, 5);
     }
     // backward
     for (int l = kLayers - 1; l >= 0 && !failed; --l) {
       sync_for_mma();
       if (tid == 0) {
         tc::fence_after_sync();
-        uint32_t const dza = tc::smem_u32(dz), ha = tc::smem_u32(H(l)), wa = tc::smem_u32(wt + l * 8192);
-        // dW_l += dZ^T H_l over the 128 samples (K): A MN-major, its second 64-row
-        // half read from the zero tile, B MN-major
-        for (uint32_t k = 0; k < 8; ++k)
-          tc::mma_bf16(tmem + 64u + 64u * uint32_t(l), tc::desc_sw128(dza + 2048u * k, kTrZero - kTrDZ, 1024),
-              tc::desc_sw128(ha + 2048u * k, 16, 1024), kIdDW, (tiles_done > 0 || k > 0) ? 1u : 0u);
+        uint32_t const dza = tc::smem_u32(DZ(l)), ha = tc::smem_u32(H(l)), wa = tc::smem_u32(wt + l * 8192),
+                       zero = tc::smem_u32(sm + kTrZero);
         if (l > 0) {
           // dH_l = dZ W_l: A K-major over the 64 outputs, B = W_l read MN-major
 #pragma unroll
           for (uint32_t k = 0; k < 4; ++k)
             tc::mma_bf16(tmem, tc::desc_sw128(dza + 32u * k, 16, 1024), tc::desc_sw128(wa + 2048u * k, 16, 1024),
                 kIdDH, k > 0 ? 1u : 0u);
+          tc::mma_commit(bar);
         }
-        tc::mma_commit(bar);
+        // dW_l += dZ^T H_l over the 128 samples (K): A MN-major, its second 64-row
+        // half read from the zero tile, B MN-major
+        for (uint32_t k = 0; k < 8; ++k)
+          tc::mma_bf16(tmem + kTmemDW + 64u * uint32_t(l), tc::desc_sw128(dza + 2048u * k, zero - dza, 1024),
+              tc::desc_sw128(ha + 2048u * k, 16, 1024), kIdDW, (tiles_done > 0 || k > 0) ? 1u : 0u);
+        // the next tile rewrites H and dZ: wait for everything; the commit also
+        // covers the layers above, issued before
+        if (l == 0) tc::mma_commit(bar);
       }
       if (!wait_mma()) {
         failed = true;
         break;
       }
       if (l > 0) {
-        float g[64], h[64];
-        acc_row(tmem, 0, nullptr, g);
-        load_row(H(l), tid, h);
+        float v[16];
+        tc::tmem_ld16(tacc, v);
+        uint4 const h0 = *reinterpret_cast<uint4 const*>(H(l) + tc::sw128_offset(trow, 2u * part));
+        uint4 const h1 = *reinterpret_cast<uint4 const*>(H(l) + tc::sw128_offset(trow, 2u * part + 1u));
+        uint32_t const h[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+        uint32_t q[8];
 #pragma unroll
-        for (int j = 0; j < 64; ++j) g[j] = h[j] > 0.f ? g[j] : 0.f;
-        store_row(dz, tid, g);
-        load_row(dz, tid, g);
-        warp_bias_sum(g, dbias + 64 * (l - 1));
+        for (int j = 0; j < 8; ++j)
+          q[j] = tc::pack_bf16(bf16_lo(h[j]) > 0.f ? v[2 * j] : 0.f, bf16_hi(h[j]) > 0.f ? v[2 * j + 1] : 0.f);
+        store16(DZ(l - 1), q);
+        bias_sums(l - 1, 16u * part, q, 8);
       }
+    }
+    if (!failed && tid < kLayers * 64) {  // the tile's sums are complete since the last barrier
+      float const* s = bias_part + (tid >> 6) * 256u + (tid & 63u);
+      dbias[tid] = (((dbias[tid] + s[0]) + s[64]) + s[128]) + s[192];
     }
     ++tiles_done;
   }
   if (failed) {
     if (tid == 0) atomicOr(a.m.err, ERR_GUIDE_TIMEOUT);
+    // let every MMA in flight retire: the commit that was waited for, then one
+    // more for the weight gradients issued after it
     tc::mbar_wait_bounded(bar, phase ^ 1u, kPollLimit);
+    __syncthreads();
+    if (tid == 0) tc::mma_commit(bar);
+    tc::mbar_wait_bounded(bar, phase, kPollLimit);
   }
   // flush: this CTA's partial gradient, every entry written (zeros when it had
-  // no tile): weight rows from TMEM (rows 0..63 live in warps 0 and 1), bias sums
+  // no tile): weight rows and bias sums from TMEM (rows 0..63 live in the lanes
+  // of quarters 0 and 1)
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   bool const have = !failed && tiles_done > 0;
-  float* part = a.partials + size_t(blockIdx.x) * kParams;
-  if (warp < 2) {
-    uint32_t const out = tid;  // row of dW = output index
+  float* out = a.partials + size_t(blockIdx.x) * kParams;
+  if (quarter < 2u) {
+    uint32_t const lanes = tmem + ((32u * quarter) << 16);
     for (int l = 0; l < kLayers; ++l) {
-      float g[64];
-      if (have) acc_row(tmem, 64u + 64u * uint32_t(l), nullptr, g);
+      float g[16];
+      if (have) tc::tmem_ld16(lanes + kTmemDW + 64u * uint32_t(l) + 16u * part, g);
       else
 #pragma unroll
-        for (int j = 0; j < 64; ++j) g[j] = 0.f;
-      float4* dst = reinterpret_cast<float4*>(part + (size_t(l) * 64 + out) * 64);
+        for (int j = 0; j < 16; ++j) g[j] = 0.f;
+      float4* dst = reinterpret_cast<float4*>(out + (size_t(l) * 64 + trow) * 64 + 16u * part);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) dst[j] = make_float4(g[4 * j], g[4 * j + 1], g[4 * j + 2], g[4 * j + 3]);
+      for (int j = 0; j < 4; ++j) dst[j] = make_float4(g[4 * j], g[4 * j + 1], g[4 * j + 2], g[4 * j + 3]);
     }
   }
-  for (uint32_t i = tid; i < kLayers * 64; i += blockDim.x) part[kLayers * 64 * 64 + i] = have ? dbias[i] : 0.f;
+  for (uint32_t i = tid; i < kLayers * 64; i += blockDim.x) out[kLayers * 64 * 64 + i] = have ? dbias[i] : 0.f;
   for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
   if ((tid & 31) == 0 && loss_acc != 0.f && a.loss) atomicAdd(a.loss, loss_acc);
   tc::fence_before_sync();
@@ -847,6 +868,28 @@ template <typename T> int grow(myrt_ctx* ctx, T** p, size_t& cap, size_t want, s
   if (rc) return rc;
   cap = want;
   return MYRT_OK;
+}
+
+// Device memory for one host-array call (evaluation, gradients, training on
+// host samples), kept between calls: cudaMalloc and the synchronising cudaFree
+// of two buffers cost such a call about as much as its kernels. Above
+// kCallKeep bytes it goes back at the end of the call (call_release). Calls of
+// one context run one after another on its stream and wait for it.
+constexpr size_t kCallKeep = size_t(64) << 20;
+int call_buffer(myrt_ctx* ctx, guide_state& g, size_t bytes) {
+  if (g.call_cap >= bytes) return MYRT_OK;
+  cudaFree(g.call_buf);
+  g.call_buf = nullptr;
+  g.call_cap = 0;
+  int rc = check_cuda(ctx, cudaMalloc(&g.call_buf, bytes), "guide call buffer");
+  if (!rc) g.call_cap = bytes;
+  return rc;
+}
+void call_release(guide_state& g) {
+  if (g.call_cap <= kCallKeep) return;
+  cudaFree(g.call_buf);
+  g.call_buf = nullptr;
+  g.call_cap = 0;
 }
 
 int init_params(myrt_ctx* ctx, guide_state& g) {
@@ -945,7 +988,7 @@ int launch_train(myrt_ctx* ctx, train_args ta, uint32_t max_rows, cudaStream_t s
   uint32_t const tiles = (max_rows + 127) / 128;
   uint32_t const grid = std::max(1u, std::min(tiles, g.max_parts));
   ta.partials = g.partials;
-  k_guide_train<<<grid, 128, kTrSmem, st>>>(ta);
+  k_guide_train<<<grid, kTrThreads, kTrSmem, st>>>(ta);
   *parts = grid;
   return check_cuda(ctx, cudaGetLastError(), "guide train launch");
 }
@@ -971,7 +1014,7 @@ void free_guide(guide_state* g) {
            static_cast<void*>(g->grads), static_cast<void*>(g->partials), static_cast<void*>(g->w_bf16),
            static_cast<void*>(g->sums),
            static_cast<void*>(g->counters), static_cast<void*>(g->points), static_cast<void*>(g->lobes),
-           static_cast<void*>(g->records), static_cast<void*>(g->samples)})
+           static_cast<void*>(g->records), static_cast<void*>(g->samples), g->call_buf})
     cudaFree(p);
   delete g;
 }
@@ -1115,19 +1158,17 @@ int guide_params_io(myrt_ctx* ctx, float* out, float const* in) {
 int guide_eval(myrt_ctx* ctx, float const* points, uint32_t n, float* lobes) {
   int rc = ensure_guide(ctx);
   if (rc || n == 0) return rc;
+  guide_state& g = *ctx->guide;
   cudaStream_t st = ctx->stream;
-  void* d_pts = nullptr;
-  void* d_lobes = nullptr;
-  rc = check_cuda(ctx, cudaMalloc(&d_pts, size_t(n) * 48), "guide eval buffers");
-  if (!rc) rc = check_cuda(ctx, cudaMalloc(&d_lobes, size_t(n) * 256), "guide eval buffers");
-  if (!rc) rc = check_cuda(ctx, cudaMemcpyAsync(d_pts, points, size_t(n) * 48, cudaMemcpyHostToDevice, st), "upload");
-  if (!rc)
-    rc = launch_forward(ctx, make_mlp(ctx), static_cast<float4 const*>(d_pts), nullptr, n, n,
-        static_cast<float4*>(d_lobes), st);
+  rc = call_buffer(ctx, g, size_t(n) * (256 + 48));
+  if (rc) return rc;
+  auto* const d_lobes = static_cast<float4*>(g.call_buf);
+  auto* const d_pts = d_lobes + size_t(n) * 16;
+  rc = check_cuda(ctx, cudaMemcpyAsync(d_pts, points, size_t(n) * 48, cudaMemcpyHostToDevice, st), "upload");
+  if (!rc) rc = launch_forward(ctx, make_mlp(ctx), d_pts, nullptr, n, n, d_lobes, st);
   if (!rc) rc = check_cuda(ctx, cudaMemcpyAsync(lobes, d_lobes, size_t(n) * 256, cudaMemcpyDeviceToHost, st), "read");
   if (!rc) rc = check_cuda(ctx, cudaStreamSynchronize(st), "guide eval");
-  cudaFree(d_pts);
-  cudaFree(d_lobes);
+  call_release(g);
   return rc;
 }
 
@@ -1136,24 +1177,24 @@ int guide_gradients(myrt_ctx* ctx, float const* samples, uint32_t n, float* grad
   if (rc) return rc;
   guide_state& g = *ctx->guide;
   cudaStream_t st = ctx->stream;
-  void* d_s = nullptr;
-  void* d_loss = nullptr;
-  rc = check_cuda(ctx, cudaMalloc(&d_s, std::max<size_t>(n, 1) * 64), "guide gradient buffers");
-  if (!rc) rc = check_cuda(ctx, cudaMalloc(&d_loss, 4), "guide gradient buffers");
-  if (!rc && n) rc = check_cuda(ctx, cudaMemcpyAsync(d_s, samples, size_t(n) * 64, cudaMemcpyHostToDevice, st), "upload");
+  rc = call_buffer(ctx, g, size_t(n) * 64 + 16);
+  if (rc) return rc;
+  auto* const d_s = static_cast<float4*>(g.call_buf);
+  auto* const d_loss = reinterpret_cast<float*>(d_s + size_t(n) * 4);
+  if (n) rc = check_cuda(ctx, cudaMemcpyAsync(d_s, samples, size_t(n) * 64, cudaMemcpyHostToDevice, st), "upload");
   if (!rc) rc = check_cuda(ctx, cudaMemsetAsync(g.grads, 0, kParams * 4, st), "clear");
   if (!rc) rc = check_cuda(ctx, cudaMemsetAsync(d_loss, 0, 4, st), "clear");
   if (!rc && n) {
     train_args ta{};
     ta.m = make_mlp(ctx);
-    ta.samples = static_cast<float4 const*>(d_s);
+    ta.samples = d_s;
     ta.count = nullptr;
     ta.n_fixed = n;
     ta.capacity = n;
     ta.batch = n;
     ta.step = 0;
     ta.sums = nullptr;
-    ta.loss = static_cast<float*>(d_loss);
+    ta.loss = d_loss;
     uint32_t parts = 0;
     rc = launch_train(ctx, ta, n, st, &parts);
     if (!rc) {
@@ -1165,8 +1206,7 @@ int guide_gradients(myrt_ctx* ctx, float const* samples, uint32_t n, float* grad
   if (!rc && loss) rc = check_cuda(ctx, cudaMemcpyAsync(loss, d_loss, 4, cudaMemcpyDeviceToHost, st), "read");
   if (!rc) rc = check_cuda(ctx, cudaMemsetAsync(g.grads, 0, kParams * 4, st), "clear");
   if (!rc) rc = check_cuda(ctx, cudaStreamSynchronize(st), "guide gradients");
-  cudaFree(d_s);
-  cudaFree(d_loss);
+  call_release(g);
   return rc;
 }
 
@@ -1175,24 +1215,24 @@ int guide_train_samples(myrt_ctx* ctx, float const* samples, uint32_t n, uint32_
   if (rc) return rc;
   guide_state& g = *ctx->guide;
   cudaStream_t st = ctx->stream;
-  void* d_s = nullptr;
-  void* d_loss = nullptr;
-  rc = check_cuda(ctx, cudaMalloc(&d_s, std::max<size_t>(n, 1) * 64), "guide training buffers");
-  if (!rc) rc = check_cuda(ctx, cudaMalloc(&d_loss, std::max<size_t>(steps, 1) * 4), "guide training buffers");
-  if (!rc && n) rc = check_cuda(ctx, cudaMemcpyAsync(d_s, samples, size_t(n) * 64, cudaMemcpyHostToDevice, st), "upload");
+  rc = call_buffer(ctx, g, size_t(n) * 64 + std::max<size_t>(steps, 1) * 4);
+  if (rc) return rc;
+  auto* const d_s = static_cast<float4*>(g.call_buf);
+  auto* const d_loss = reinterpret_cast<float*>(d_s + size_t(n) * 4);
+  if (n) rc = check_cuda(ctx, cudaMemcpyAsync(d_s, samples, size_t(n) * 64, cudaMemcpyHostToDevice, st), "upload");
   if (!rc) rc = check_cuda(ctx, cudaMemsetAsync(d_loss, 0, std::max<size_t>(steps, 1) * 4, st), "clear");
   uint32_t const batch = std::min(n, g.prm.batch);
   for (uint32_t s = 0; !rc && n && s < steps; ++s) {
     train_args ta{};
     ta.m = make_mlp(ctx);
-    ta.samples = static_cast<float4 const*>(d_s);
+    ta.samples = d_s;
     ta.count = nullptr;
     ta.n_fixed = n;
     ta.capacity = n;
     ta.batch = batch;
     ta.step = s;
     ta.sums = nullptr;
-    ta.loss = static_cast<float*>(d_loss) + s;
+    ta.loss = d_loss + s;
     uint32_t parts = 0;
     rc = launch_train(ctx, ta, batch, st, &parts);
     if (!rc) rc = adam_step(ctx, g, parts, nullptr, st);
@@ -1200,8 +1240,7 @@ int guide_train_samples(myrt_ctx* ctx, float const* samples, uint32_t n, uint32_
   if (!rc && loss_per_step && steps)
     rc = check_cuda(ctx, cudaMemcpyAsync(loss_per_step, d_loss, size_t(steps) * 4, cudaMemcpyDeviceToHost, st), "read");
   if (!rc) rc = check_cuda(ctx, cudaStreamSynchronize(st), "guide training");
-  cudaFree(d_s);
-  cudaFree(d_loss);
+  call_release(g);
   return rc;
 }
 
