@@ -92,27 +92,88 @@ __device__ __forceinline__ float normpdf3(float3 v, float sigma) {
   float const d = (v.x * v.x + v.y * v.y) + v.z * v.z;
   return 0.39894f * myrt_glmath::exp((-0.5f * d) / (sigma * sigma)) / sigma;
 }
-__global__ void k_pp_denoise(pass_args a) {
-  int const x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+// The pass is arithmetic: 81 exponentials and 162 divisions per pixel on cached
+// texels. A block keeps its texels and their halo in shared memory, clamped
+// once; the spatial weights are computed once per block; the two divisors are
+// the same for the whole pass, so the quotients come from their reciprocals
+// and two remainder corrections (div_by); the exponential of a non-positive
+// argument rounds with a constant added and subtracted (exp_neg) instead of
+// the quarter-rate conversions. Weights below e^-50, where remainders could
+// leave the float range, and divisors far from 1 (FAST = false) take the plain
+// expressions, as do infinities and NaN. Every result equals the plain
+// expressions' bit for bit. 2048 x 2048: 1,059 -> 580 us.
+//
+// x / b for r = 1 / b rounded to nearest: after one correction the quotient is
+// within an ulp, and a second one with the exact remainder rounds it correctly
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34, 1990).
+__device__ __forceinline__ float div_by(float q, float x, float b, float r) {  // q = x r
+  q = __fmaf_rn(__fmaf_rn(-q, b, x), r, q);
+  return __fmaf_rn(__fmaf_rn(-q, b, x), r, q);
+}
+// myrt_glmath::exp for -60 < x <= 0: the same operations, n = rint(x log2 e) by
+// adding and subtracting 1.5 * 2^23, 2^n from the sum's low bits.
+__device__ __forceinline__ float exp_neg(float x) {
+  float const th = x * myrt_glmath::kLog2e_hi;
+  float const tl = __fmaf_rn(x, myrt_glmath::kLog2e_lo, __fmaf_rn(x, myrt_glmath::kLog2e_hi, -th));
+  float const t = th + 12582912.f;
+  float const f = (th - (t - 12582912.f)) + tl;
+  return myrt_glmath::exp2_kernel(f) * __uint_as_float((__float_as_uint(t) << 23) + 0x3f800000u);
+}
+constexpr int kDenW = 32, kDenH = 8, kDenHalo = 4, kDenPitch = kDenW + 2 * kDenHalo;
+struct denoise_div {
+  float s2, r_s2;  // sigma^2 of the range weight and its reciprocal
+  float s, r_s;    // sigma
+};
+template <bool FAST>
+__global__ void __launch_bounds__(kDenW* kDenH) k_pp_denoise(pass_args a, denoise_div dv) {
+  __shared__ float4 s_tex[(kDenH + 2 * kDenHalo) * kDenPitch];
+  __shared__ float s_kernel[kDenHalo + 1], s_bz;
+  int const x0 = blockIdx.x * kDenW, y0 = blockIdx.y * kDenH;
+  int const t = threadIdx.y * kDenW + threadIdx.x;
+  if (t <= kDenHalo) s_kernel[t] = normpdf(float(t), a.p[0]);
+  else if (t == 32) s_bz = 1.f / normpdf(0.f, a.p[1]);
+  for (int i = t; i < (kDenH + 2 * kDenHalo) * kDenPitch; i += kDenW * kDenH) {
+    int const sx = min(max(x0 + i % kDenPitch - kDenHalo, 0), a.in.w - 1);
+    int const sy = min(max(y0 + i / kDenPitch - kDenHalo, 0), a.in.h - 1);
+    float4 const v = a.in.p[size_t(sy) * a.in.w + sx];
+    s_tex[i] = make_float4(fminf(fmaxf(v.x, 0.f), 1.f), fminf(fmaxf(v.y, 0.f), 1.f), fminf(fmaxf(v.z, 0.f), 1.f), 0.f);
+  }
+  __syncthreads();
+  int const x = x0 + threadIdx.x, y = y0 + threadIdx.y;
   if (x >= a.ow || y >= a.oh) return;
-  constexpr int kSize = 4;
-  float kernel[2 * kSize + 1];
-  for (int j = 0; j <= kSize; ++j) kernel[kSize + j] = kernel[kSize - j] = normpdf(float(j), a.p[0]);
-  float4 const c4 = fetch(a.in, x, y);
-  float3 const c{c4.x, c4.y, c4.z};
+  float4 const c = a.in.p[size_t(y) * a.in.w + x];
+  float kernel[kDenHalo + 1];
+  for (int j = 0; j <= kDenHalo; ++j) kernel[j] = s_kernel[j];
+  float const bZ = s_bz;
   float Z = 0.f;
   float3 fc{0.f, 0.f, 0.f};
-  float const bZ = 1.f / normpdf(0.f, a.p[1]);
-  for (int i = -kSize; i <= kSize; ++i)
-    for (int j = -kSize; j <= kSize; ++j) {
-      int const sx = min(max(x + i, 0), a.in.w - 1), sy = min(max(y + j, 0), a.in.h - 1);
-      float4 const t = fetch(a.in, sx, sy);
-      float3 const cc{fminf(fmaxf(t.x, 0.f), 1.f), fminf(fmaxf(t.y, 0.f), 1.f), fminf(fmaxf(t.z, 0.f), 1.f)};
-      float const factor =
-          ((normpdf3(float3{cc.x - c.x, cc.y - c.y, cc.z - c.z}, a.p[1]) * bZ) * kernel[kSize + j]) * kernel[kSize + i];
+#pragma unroll 1
+  for (int i = -kDenHalo; i <= kDenHalo; ++i) {
+    float4 const* col = s_tex + threadIdx.y * kDenPitch + threadIdx.x + kDenHalo + i;
+    float const ki = s_kernel[i < 0 ? -i : i];
+#pragma unroll
+    for (int j = -kDenHalo; j <= kDenHalo; ++j) {
+      float4 const cc = col[(j + kDenHalo) * kDenPitch];
+      float3 const v{cc.x - c.x, cc.y - c.y, cc.z - c.z};
+      float pdf;
+      if (FAST) {
+        float const e = -0.5f * ((v.x * v.x + v.y * v.y) + v.z * v.z);
+        float const q = e * dv.r_s2;
+        if (q >= -50.f) {
+          float const w = 0.39894f * exp_neg(div_by(q, e, dv.s2, dv.r_s2));
+          pdf = div_by(w * dv.r_s, w, dv.s, dv.r_s);
+        } else {
+          pdf = normpdf3(v, a.p[1]);
+        }
+      } else {
+        pdf = normpdf3(v, a.p[1]);
+      }
+      float const factor = ((pdf * bZ) * kernel[j < 0 ? -j : j]) * ki;
       Z += factor;
       fc.x += factor * cc.x, fc.y += factor * cc.y, fc.z += factor * cc.z;
     }
+  }
   a.out[size_t(y) * a.ow + x] = store16(make_float4(fc.x / Z, fc.y / Z, fc.z / Z, 1.f));
 }
 
@@ -121,18 +182,50 @@ __constant__ float kBlur[16] = {0.08756118061424645f, 0.08547984344465417f, 0.07
     0.0705164133185798f, 0.05958841266910679f, 0.04798885898065629f, 0.03683205838316095f, 0.0269412473017388f,
     0.018780823225920923f, 0.012477173150624141f, 0.007899915153736418f, 0.004766876346593609f,
     0.0027412691146821303f, 0.001502371210393176f, 0.0007847156649807812f, 0.0003906237796399568f};
-__global__ void k_pp_blur(pass_args a) {
+// One axis of a bilinear sample (bilinear, mirrored): the two texels and the
+// weight of the second.
+struct axis_tap {
+  int i0, i1;
+  float a;
+};
+__device__ __forceinline__ axis_tap tap_of(float s, int size) {
+  float const u = s * float(size) - 0.5f;
+  float const fu = floorf(u);
+  int const i = int(fu);
+  return {mirror_repeat(i, size), mirror_repeat(i + 1, size), u - fu};
+}
+// Taps move along one axis, so the other axis' texels and weight are found once
+// per pixel. The samples are bilinear()'s bit for bit. Issue-bound (82 % of the
+// slots, 95 % of the reads hit L1); keeping the last texel for the next tap
+// made no difference. A 1024 x 1024 pass: 113 -> 100 us along x, 112 -> 91 along y.
+template <bool ALONG_Y> __global__ void __launch_bounds__(256) k_pp_blur(pass_args a) {
   int const x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= a.ow || y >= a.oh) return;
   float const ix = 1.f / float(a.in.w), iy = 1.f / float(a.in.h);
   float const px = float(x), py = float(y);
-  float4 r = f4mul(kBlur[0], bilinear(a.in, px * ix, py * iy, true));
-  int const dir = a.i0 != 0 ? 1 : 0;
-  float const sx = float(1 - dir) * a.p[0], sy = float(dir) * a.p[0];
+  axis_tap const fix = ALONG_Y ? tap_of(px * ix, a.in.w) : tap_of(py * iy, a.in.h);
+  int const size = ALONG_Y ? a.in.h : a.in.w;
+  float const p0 = ALONG_Y ? py : px, inv = ALONG_Y ? iy : ix;
+  // texels at position i of the moving axis, at the fixed axis' two places
+  auto texel = [&](int i, int f) {
+    return ALONG_Y ? a.in.p[size_t(i) * a.in.w + f] : a.in.p[size_t(f) * a.in.w + i];
+  };
+  auto sample = [&](float pos) {
+    axis_tap const m = tap_of(pos * inv, size);
+    float4 const n0 = texel(m.i0, fix.i0), n1 = texel(m.i0, fix.i1);
+    float4 const f0 = texel(m.i1, fix.i0), f1 = texel(m.i1, fix.i1);
+    // w00 t00 + w10 t10 + w01 t01 + w11 t11, x before y
+    float const ax = ALONG_Y ? fix.a : m.a, ay = ALONG_Y ? m.a : fix.a;
+    float const w00 = (1.f - ax) * (1.f - ay), w10 = ax * (1.f - ay), w01 = (1.f - ax) * ay, w11 = ax * ay;
+    float4 const t10 = ALONG_Y ? n1 : f0, t01 = ALONG_Y ? f0 : n1;
+    return f4add(f4add(f4add(f4mul(w00, n0), f4mul(w10, t10)), f4mul(w01, t01)), f4mul(w11, f1));
+  };
+  float4 r = f4mul(kBlur[0], sample(p0));
+#pragma unroll 3
   for (int i = 1; i < 16; ++i) {
-    float const fi = float(i);
-    float4 const s0 = bilinear(a.in, (px + fi * sx) * ix, (py + fi * sy) * iy, true);
-    float4 const s1 = bilinear(a.in, (px - fi * sx) * ix, (py - fi * sy) * iy, true);
+    float const off = float(i) * a.p[0];
+    float4 const s0 = sample(p0 + off);
+    float4 const s1 = sample(p0 - off);
     r = f4add(r, f4mul(kBlur[i], f4add(s0, s1)));
   }
   a.out[size_t(y) * a.ow + x] = store16(r);
@@ -251,8 +344,19 @@ extern "C" int myrt_post_pass(myrt_ctx* ctx, myrt_pp_pass const* pass, myrt_imag
   dim3 const block(16, 16);
   dim3 const grid((out->width + 15) / 16, (out->height + 15) / 16);
   switch (pass->op) {
-    case MYRT_PP_DENOISE: k_pp_denoise<<<grid, block, 0, st>>>(a); break;
-    case MYRT_PP_BLUR: k_pp_blur<<<grid, block, 0, st>>>(a); break;
+    case MYRT_PP_DENOISE: {
+      float const s = a.p[1], s2 = s * s;
+      denoise_div const dv{s2, 1.f / s2, s, 1.f / s};
+      dim3 const db(kDenW, kDenH), dg((out->width + kDenW - 1) / kDenW, (out->height + kDenH - 1) / kDenH);
+      // div_by needs quotients, remainders and reciprocals well inside the float range
+      if (s2 >= 0x1p-60f && s2 <= 0x1p60f) k_pp_denoise<true><<<dg, db, 0, st>>>(a, dv);
+      else k_pp_denoise<false><<<dg, db, 0, st>>>(a, dv);
+      break;
+    }
+    case MYRT_PP_BLUR:
+      if (a.i0 != 0) k_pp_blur<true><<<grid, block, 0, st>>>(a);
+      else k_pp_blur<false><<<grid, block, 0, st>>>(a);
+      break;
     case MYRT_PP_CUTOFF: k_pp_cutoff<<<grid, block, 0, st>>>(a); break;
     case MYRT_PP_ADD: k_pp_add<<<grid, block, 0, st>>>(a); break;
     case MYRT_PP_TONEMAP: k_pp_tonemap<<<grid, block, 0, st>>>(a); break;
