@@ -157,13 +157,17 @@ typedef struct myrt_tuning {
                                 1 = device linear BVH (Morton order, radix tree, 8-wide collapse on the
                                 GPU): milliseconds for millions of triangles, slower traversal */
   uint32_t trace_order;      /* visiting order of closest / any-hit batches: 0 = device-memory queries
-                                of at least 1 Mi rays sorted by origin and direction cell, host-memory
-                                queries in input order; 1 = input order; 2 = always sorted. The
-                                trace passes of reference shading likewise: 0 = the first two passes
-                                sorted once the frames in flight hold 1 Mi rays, 1 = never, 2 = every
-                                pass; and the extension queues of physical / guided waves: 0 = those
-                                of vertices 1 and 2 in waves of at least 1 Mi paths, 1 = never, 2 =
-                                every vertex after the camera's. Results never depend on it. */
+                                of at least 1 Mi rays by origin and direction cell (warps of 32
+                                neighbouring rays that share their cells already, camera rays for
+                                one, stay together), host-memory queries in input order; 1 = input
+                                order; 2 = always by cell. The trace passes of reference shading
+                                likewise: 0 = the first two bounces' rays and the first two passes'
+                                shadow rays once the frames in flight hold 1 Mi rays, 1 = never, 2 =
+                                every pass; and the extension queues of physical / guided waves: 0 =
+                                those of vertices 1 to 3 in waves of at least 1 Mi paths, 1 = never,
+                                2 = every vertex after the camera's. Without device memory for the
+                                order (12 bytes a ray and 32 MB), input order. Results never depend
+                                on it. */
   uint32_t sdf_cells;        /* myrt_sdf_upload: cells along the longest axis of the grid of
                                 instruction segments built for each program that is a tree of
                                 unions / smooth unions over translated spheres, boxes, tori and

@@ -10,7 +10,6 @@
 #include <string>
 #include <vector>
 
-#include <cub/device/device_radix_sort.cuh>
 
 #include "../../include/myrt_cuda.h"
 #include "bvh8.hpp"
@@ -127,22 +126,19 @@ int launch_persistent(myrt_ctx* ctx, trace_args const& a, cudaStream_t s) {
   return MYRT_OK;
 }
 
-constexpr uint32_t kOrderMin = 1u << 20;  // batches from this size on are sorted (trace_order 0)
-
-void free_order(myrt_ctx::order_scratch& o) {
-  for (int k = 0; k < 2; ++k) {
-    cudaFree(o.keys[k]);
-    cudaFree(o.vals[k]);
-    o.keys[k] = o.vals[k] = nullptr;
+// The cell of ray i of a batch given as (o, tmin), (d, tmax) float4 pairs.
+struct batch_cell {
+  float4 const* rays;
+  float3 lo, scale;
+  __device__ uint32_t operator()(uint32_t i) const {
+    return ray_cell(__ldg(rays + 2 * size_t(i)), __ldg(rays + 2 * size_t(i) + 1), lo, scale);
   }
-  cudaFree(o.temp);
-  o.temp = nullptr;
-  o.cap = o.temp_bytes = 0;
-}
+};
 
-// Sorts the batch's ray indices by origin / direction cell (rayorder.cuh) into
-// the lane's scratch and points a.perm at the order. The scratch of a lane is
-// reused by later queries on any stream: each use waits for the previous one.
+// The batch's visiting order (rayorder.cuh) into the lane's scratch and a.perm;
+// input order (a.perm null) when the device has no room for it. The scratch of
+// a lane is reused by later queries on any stream: each use waits for the
+// previous one.
 int order_rays(myrt_ctx* ctx, trace_args& a, int lane, cudaStream_t s) {
   auto& o = ctx->order[lane];
   if (!o.done) {
@@ -151,38 +147,12 @@ int order_rays(myrt_ctx* ctx, trace_args& a, int lane, cudaStream_t s) {
   }
   int rc = check_cuda(ctx, cudaStreamWaitEvent(s, o.done, 0), "ray order wait");
   if (rc) return rc;
-  size_t need = 0;
-  rc = check_cuda(ctx, cub::DeviceRadixSort::SortPairs(nullptr, need, o.keys[0], o.keys[1], o.vals[0], o.vals[1],
-                           int(a.n), 0, kOrderKeyBits, s), "ray order size");
-  if (rc) return rc;
-  if (o.cap < a.n || o.temp_bytes < need) {
-    rc = check_cuda(ctx, cudaStreamSynchronize(s), "ray order realloc");
-    if (rc) return rc;
-    free_order(o);
-    size_t const cap = std::max<size_t>(a.n, o.cap);
-    for (int k = 0; k < 2 && !rc; ++k) {
-      rc = check_cuda(ctx, cudaMalloc(reinterpret_cast<void**>(&o.keys[k]), cap * 4), "ray order keys");
-      if (!rc) rc = check_cuda(ctx, cudaMalloc(reinterpret_cast<void**>(&o.vals[k]), cap * 4), "ray order indices");
-    }
-    if (!rc) rc = check_cuda(ctx, cudaMalloc(&o.temp, need), "ray order temporary");
-    if (rc) {
-      free_order(o);
-      return rc;
-    }
-    o.cap = cap;
-    o.temp_bytes = need;
-  }
-  float3 lo, sc;
-  ray_key_grid(ctx->scene.bounds, lo, sc);
-  k_ray_keys<<<(a.n + 255) / 256, 256, 0, s>>>(a.rays, a.n, lo, sc, o.keys[0], o.vals[0]);
-  rc = check_cuda(ctx, cudaGetLastError(), "ray key launch");
-  if (rc) return rc;
-  size_t tb = o.temp_bytes;
-  rc = check_cuda(ctx, cub::DeviceRadixSort::SortPairs(o.temp, tb, o.keys[0], o.keys[1], o.vals[0], o.vals[1],
-                           int(a.n), 0, kOrderKeyBits, s), "ray order sort");
-  if (rc) return rc;
-  a.perm = o.vals[1];
-  return MYRT_OK;
+  if (!ensure_ray_order(o.order, a.n, s)) return MYRT_OK;
+  batch_cell cell{a.rays, {}, {}};
+  ray_cell_grid(ctx->scene.bounds, cell.lo, cell.scale);
+  rc = check_cuda(ctx, build_ray_order(o.order, cell, a.n, nullptr, s), "ray order launch");
+  if (!rc) a.perm = o.order.dev.perm;
+  return rc;
 }
 
 int launch_trace_kernels(myrt_ctx* ctx, trace_args a, int intersector, bool any, bool stats, cudaStream_t s);
@@ -469,7 +439,7 @@ int myrt_ctx_destroy(myrt_ctx* ctx) {
   ctx->guide = nullptr;
   for (auto& p : ctx->stage) cudaFree(p);
   for (auto& o : ctx->order) {
-    free_order(o);
+    free_ray_order(o.order);
     if (o.done) cudaEventDestroy(o.done);
   }
   for (auto* list : {&ctx->phase_pending, &ctx->phase_pool})

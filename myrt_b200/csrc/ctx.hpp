@@ -98,6 +98,20 @@ struct device_sdf {
   int n_programs = 0;
 };
 
+// Scratch of a visiting order (rayorder.cuh); 12 bytes per slot and 32 MB.
+struct ray_order_dev {
+  uint32_t* count = nullptr;   // rays per cell, zero between uses
+  uint32_t* offset = nullptr;  // first position of a cell's rays
+  uint2* rec = nullptr;        // (cell, rank) of every ray of the warps taken apart
+  uint32_t* warp = nullptr;    // those warps' first slots
+  uint32_t* perm = nullptr;    // the order: slot of the i-th thread
+  uint32_t* ctr = nullptr;     // warps taken apart, rays of the others, positions given out
+};
+struct ray_order {
+  ray_order_dev dev;
+  size_t cap = 0;  // slots
+};
+
 // Wavefront render state (sequential_pathtracer's buffers and counters).
 struct render_state {
   uint32_t width = 0, height = 0;
@@ -110,11 +124,8 @@ struct render_state {
   float* pass_tex = nullptr;            // frames * passes * 1024 random texture floats
   float4* fcol = nullptr;               // frames in flight: final colour per frame and pixel
   uint32_t frames_cap = 0;              // frames in flight the ray buffers hold
-  uint32_t* okeys[2] = {nullptr, nullptr};  // visiting order of a trace pass: keys, slots
-  uint32_t* ovals[2] = {nullptr, nullptr};
-  void* otemp = nullptr;                // radix sort temporary
+  ray_order order;                      // visiting order of a trace pass
   float4* shadow_q = nullptr;           // NEE shadow rays of a trace pass, 2 float4 each
-  size_t otemp_bytes = 0;
   size_t pass_tex_capacity = 0;         // in floats
   uint32_t sample_counter = 0;          // frames accumulated since the last reset
   int64_t pending_first = -1;           // myrt_begin_samples: first sample index of the next render
@@ -134,10 +145,7 @@ struct physical_state {
   float4* shadow = nullptr;             // 3 float4 per shadow ray: (o, path), (d, tmax), (contribution, -)
   float4* radiance = nullptr;           // per path: rgb
   uint32_t* counts = nullptr;           // [0..1] ray queues, [2] shadow queue
-  uint32_t* okeys[2] = {nullptr, nullptr};  // visiting order of an extension queue: keys, entries
-  uint32_t* ovals[2] = {nullptr, nullptr};
-  void* otemp = nullptr;                // radix sort temporary
-  size_t otemp_bytes = 0;
+  ray_order order;                      // visiting order of an extension queue
   unsigned long long* stats = nullptr;  // paths, extension rays, shadow rays (cumulative)
   void* lights = nullptr;               // ps::area_light[n_lights]
   int n_lights = 0;
@@ -170,13 +178,9 @@ struct myrt_ctx {
   // staging buffers of the host-memory entry points (one chunk slot per lane)
   void* stage[4] = {nullptr, nullptr, nullptr, nullptr};
   size_t stage_bytes = 0;
-  // ray-order scratch per stream lane (keys and indices, double-buffered, and
-  // the radix sort's temporary storage); `done` orders reuse across streams
+  // ray-order scratch per stream lane; `done` orders reuse across streams
   struct order_scratch {
-    uint32_t* keys[2] = {nullptr, nullptr};
-    uint32_t* vals[2] = {nullptr, nullptr};
-    void* temp = nullptr;
-    size_t cap = 0, temp_bytes = 0;
+    myrt_b200::ray_order order;
     cudaEvent_t done = nullptr;
   } order[4];
   // reference-mode textures (slots) and environment cube map; d_textures

@@ -30,8 +30,6 @@
 // Compiled with -fmad=false (build.py) like the other shading unit.
 #include <cuda_runtime.h>
 
-#include <cub/device/device_radix_sort.cuh>
-
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -72,7 +70,7 @@ struct pt_scene {
   ps::area_light const* lights;
   int n_lights;
   sdfk::sdf_dev sdf;  // steps / eps come from the job
-  float3 key_lo, key_scale;  // ray_key's grid over the scene box
+  float3 key_lo, key_scale;  // ray_cell's grid over the scene box
 };
 
 // One job within one wave.
@@ -242,21 +240,16 @@ __global__ void __launch_bounds__(kPtBlock, MINB) k_pt_extend(pt_wave w, int v, 
   }
 }
 
-// Visiting order of an extension queue: each live entry's origin / direction
-// cell key in its scene's grid (ray_key), 0xFFFFFF (after every live key) for
-// the wave's empty slots.
-__global__ void __launch_bounds__(256) k_pt_keys(pt_wave w, float4 const* __restrict__ q,
-    uint32_t const* __restrict__ count, uint32_t n_max, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-  uint32_t const i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_max) return;
-  uint32_t key = 0xFFFFFFu;
-  if (i < *count) {
+// Visiting order of an extension queue: an entry's cell in its scene's grid
+// (rayorder.cuh).
+struct queue_cell {
+  pt_wave w;
+  float4 const* q;
+  __device__ uint32_t operator()(uint32_t i) const {
     pt_scene const& s = w.scenes[w.jobs[__float_as_int(q[3 * size_t(i) + 2].w)].scene];
-    key = min(ray_key(q[3 * size_t(i)], q[3 * size_t(i) + 1], s.key_lo, s.key_scale), 0xFFFFFEu);
+    return ray_cell(q[3 * size_t(i)], q[3 * size_t(i) + 1], s.key_lo, s.key_scale);
   }
-  keys[i] = key;
-  vals[i] = i;
-}
+};
 
 // ---- shade ------------------------------------------------------------------------------
 struct shade_io {
@@ -507,17 +500,15 @@ void mat_mul4(float const* a, float const* b, float* out) {
 }
 
 int ensure_queues(myrt_ctx* ctx, physical_state& P, size_t paths) {
+  // without room for the visiting order the queues are visited as they are
+  uint32_t const order = ctx->tuning.trace_order;
+  if (order == 2 || (order == 0 && paths >= kOrderMin)) ensure_ray_order(P.order, paths, ctx->stream);
   if (P.capacity >= paths && P.queue[0]) return MYRT_OK;
   for (void* p : {static_cast<void*>(P.queue[0]), static_cast<void*>(P.queue[1]), static_cast<void*>(P.hits),
-           static_cast<void*>(P.shadow), static_cast<void*>(P.radiance), static_cast<void*>(P.counts),
-           static_cast<void*>(P.okeys[0]), static_cast<void*>(P.okeys[1]), static_cast<void*>(P.ovals[0]),
-           static_cast<void*>(P.ovals[1]), P.otemp})
+           static_cast<void*>(P.shadow), static_cast<void*>(P.radiance), static_cast<void*>(P.counts)})
     cudaFree(p);
   P.queue[0] = P.queue[1] = P.hits = P.shadow = P.radiance = nullptr;
   P.counts = nullptr;
-  P.okeys[0] = P.okeys[1] = P.ovals[0] = P.ovals[1] = nullptr;
-  P.otemp = nullptr;
-  P.otemp_bytes = 0;
   P.capacity = 0;
   int rc = MYRT_OK;
   auto alloc = [&](void** p, size_t bytes, char const* what) {
@@ -529,14 +520,6 @@ int ensure_queues(myrt_ctx* ctx, physical_state& P, size_t paths) {
   alloc(reinterpret_cast<void**>(&P.shadow), paths * 48, "shadow queue");
   alloc(reinterpret_cast<void**>(&P.radiance), paths * 16, "path radiance");
   alloc(reinterpret_cast<void**>(&P.counts), 4 * sizeof(uint32_t), "queue counts");
-  for (int k = 0; k < 2; ++k) {  // visiting order of the extension queues
-    alloc(reinterpret_cast<void**>(&P.okeys[k]), paths * 4, "queue order keys");
-    alloc(reinterpret_cast<void**>(&P.ovals[k]), paths * 4, "queue order entries");
-  }
-  if (!rc)
-    rc = check_cuda(ctx, cub::DeviceRadixSort::SortPairs(nullptr, P.otemp_bytes, P.okeys[0], P.okeys[1], P.ovals[0],
-                             P.ovals[1], int(paths), 0, kOrderKeyBits, ctx->stream), "queue order size");
-  alloc(&P.otemp, std::max<size_t>(P.otemp_bytes, 16), "queue order temporary");
   if (!rc && !P.stats) {
     alloc(reinterpret_cast<void**>(&P.stats), 4 * sizeof(unsigned long long), "ray statistics");
     if (!rc) rc = check_cuda(ctx, cudaMemsetAsync(P.stats, 0, 4 * sizeof(unsigned long long), ctx->stream), "clear");
@@ -556,7 +539,7 @@ pt_scene scene_of(myrt_ctx const* ctx) {
           ctx->sdf.cell_list, ctx->sdf.op_count, ctx->sdf.cell_outer, ctx->sdf.chain_hdr, ctx->sdf.chain_rec, ctx->sdf.chain_start,
           ctx->sdf.chain_list},
       float3{0.f, 0.f, 0.f}, float3{0.f, 0.f, 0.f}};
-  ray_key_grid(S.bounds, r.key_lo, r.key_scale);
+  ray_cell_grid(S.bounds, r.key_lo, r.key_scale);
   return r;
 }
 
@@ -672,22 +655,19 @@ int launch_plan(myrt_ctx* ctx, physical_state& P, cudaStream_t st, pt_scene cons
     int cur = 0;
     for (int v = 0; v <= wp.max_depth; ++v) {
       bool const last = v == wp.max_depth;
-      // visiting order (trace_order): the first bounces' queues (vertices 1 and 2), whose paths have
-      // scattered, sorted by origin / direction cell in waves of at least 1 Mi paths (0); never (1);
-      // every vertex after the camera's (2). Results never depend on it.
+      // visiting order (trace_order): the first bounces' queues (vertices 1 to 3), whose paths have
+      // scattered, by origin / direction cell in waves of at least 1 Mi paths (0); never (1); every
+      // vertex after the camera's (2). Results never depend on it. 512x512, 64 spp: vertex 1 alone
+      // 23.7, 1 and 2 23.1, 1 to 3 22.8, 1 to 5 23.0 ms; the shadow queues too: no difference.
       uint32_t const order = ctx->tuning.trace_order;
-      bool const sorted = per_entry && v >= 1 && wp.n_paths <= P.capacity &&
-          (order == 2 || (order == 0 && v <= 2 && wp.n_paths >= (1u << 20)));
-      uint32_t const* perm = nullptr;
+      bool const sorted = per_entry && v >= 1 && wp.n_paths <= P.order.cap &&
+          (order == 2 || (order == 0 && v <= 3 && wp.n_paths >= kOrderMin));
       if (sorted) {
-        k_pt_keys<<<(wp.n_paths + 255) / 256, 256, 0, st>>>(w, P.queue[cur], P.counts + cur, wp.n_paths, P.okeys[0],
-            P.ovals[0]);
-        size_t tb = P.otemp_bytes;
-        int rc = check_cuda(ctx, cub::DeviceRadixSort::SortPairs(P.otemp, tb, P.okeys[0], P.okeys[1], P.ovals[0],
-                                     P.ovals[1], int(wp.n_paths), 0, kOrderKeyBits, st), "queue order sort");
+        int rc = check_cuda(ctx, build_ray_order(P.order, queue_cell{w, P.queue[cur]}, wp.n_paths, P.counts + cur, st),
+            "queue order");
         if (rc) return rc;
-        perm = P.ovals[1];
       }
+      uint32_t const* const perm = sorted ? P.order.dev.perm : nullptr;
       if (any_sdf)
         k_pt_extend<true><<<qgrid, kPtBlock, 0, st>>>(w, v, P.queue[cur], P.counts + cur, P.hits,
             P.counts + (1 - cur), P.counts + 2, P.stats, perm);
@@ -744,9 +724,9 @@ int grow_bytes(myrt_ctx* ctx, void** p, size_t& cap, size_t bytes, char const* w
 void free_physical(physical_state& P) {
   for (void* p : {static_cast<void*>(P.queue[0]), static_cast<void*>(P.queue[1]), static_cast<void*>(P.hits),
            static_cast<void*>(P.shadow), static_cast<void*>(P.radiance), static_cast<void*>(P.counts), P.lights,
-           static_cast<void*>(P.stats), P.tables, static_cast<void*>(P.okeys[0]), static_cast<void*>(P.okeys[1]),
-           static_cast<void*>(P.ovals[0]), static_cast<void*>(P.ovals[1]), P.otemp})
+           static_cast<void*>(P.stats), P.tables})
     cudaFree(p);
+  free_ray_order(P.order);
   P = physical_state{};
 }
 

@@ -9,7 +9,7 @@
 //                  rays k_trace_pass leaves, so that every lane walks one
 //   k_color_pass   pt_color.comp:77-202 (sky gradient, no cubemap), plus a
 //                  per-block count of surviving rays for the compaction
-//   k_gen_keys     visiting order of the first two trace passes (ray_key)
+//   rayorder.cuh   visiting order of the first two trace passes
 //   k_resolve_frames  the frames in flight into the accumulation, in order
 //   k_scan_blocks + k_scatter
 //                  pt_ray_filter.comp:49-64 as a STABLE compaction: survivors
@@ -42,7 +42,6 @@
 #include <random>
 #include <vector>
 
-#include <cub/device/device_radix_sort.cuh>
 
 #include "../../include/myrt_cuda.h"
 #include "ctx.hpp"
@@ -190,6 +189,29 @@ __global__ void __launch_bounds__(kBlock) k_generate(uint32_t W, uint32_t H, uin
   g[4] = make_float4(1.f, 1.f, 0.f, 0.f);
 }
 
+// Visiting order of a trace pass over the frames in flight: the cell of the ray
+// slot of thread t of the pass's grid (rayorder.cuh).
+struct pass_cell {
+  float4 const* gen;
+  uint32_t const* count;
+  uint32_t slots, nb;
+  float3 lo, scale;
+  __device__ uint32_t operator()(uint32_t t) const {
+    uint32_t const f = t / (nb * kBlock), id = t - f * nb * kBlock;
+    if (id >= count[f]) return kOrderCells;
+    float4 const* g = gen + 5 * (size_t(f) * slots + id);
+    return ray_cell(g[0], g[1], lo, scale);
+  }
+};
+// The same of a queue of shadow rays.
+struct shadow_cell {
+  float4 const* q;
+  float3 lo, scale;
+  __device__ uint32_t operator()(uint32_t i) const {
+    return ray_cell(q[2 * size_t(i)], q[2 * size_t(i) + 1], lo, scale);
+  }
+};
+
 // ---- pt_trace.comp --------------------------------------------------------------
 // One thread per ray of the pass. The steps are ordered so that little state
 // is live across the two tree walks: the closest-hit walk needs only the ray;
@@ -198,23 +220,6 @@ __global__ void __launch_bounds__(kBlock) k_generate(uint32_t W, uint32_t H, uin
 // follow them as in the reference; the trace record is written before the
 // shadow walk, which then only adds the light term. Same operations, same
 // results as the reference's order.
-// Visiting order of a trace pass over the frames in flight: for every thread
-// of the pass's grid, the origin / direction cell key of its ray slot
-// (ray_key), or 0xFFFFFF, after every live key, for an empty slot.
-__global__ void __launch_bounds__(kBlock) k_gen_keys(float4 const* __restrict__ gen, uint32_t const* __restrict__ count,
-    uint32_t slots, uint32_t nb, float3 lo, float3 cell_scale, uint32_t* __restrict__ keys,
-    uint32_t* __restrict__ vals) {
-  frame_slot const fs = frame_of(nb);
-  uint32_t const t = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t key = 0xFFFFFFu;
-  if (fs.id < count[fs.f]) {
-    float4 const* g = gen + 5 * (size_t(fs.f) * slots + fs.id);
-    key = min(ray_key(g[0], g[1], lo, cell_scale), 0xFFFFFEu);
-  }
-  keys[t] = key;
-  vals[t] = t;
-}
-
 // gen / trace: the frames' regions of `slots` rays; count[f]: frame f's rays.
 // perm (may be null): thread t takes the ray slot of thread perm[t] of the grid.
 // shadow_q (may be null): without SDF drawables, the NEE shadow rays are
@@ -379,9 +384,10 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_pass(scene_dev s, pass_rand
 // trace record, as k_trace_pass computes it in place.
 constexpr int kShadowBlock = 128;
 __global__ void __launch_bounds__(kShadowBlock, 8) k_shadow_pass(scene_dev s, float4 const* __restrict__ q,
-    uint32_t const* __restrict__ count, float4* __restrict__ trace) {
-  uint32_t const i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t const* __restrict__ count, float4* __restrict__ trace, uint32_t const* __restrict__ perm) {
+  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= *count) return;
+  if (perm) i = __ldg(perm + i);
   float4 const a = q[2 * size_t(i)], b = q[2 * size_t(i) + 1];
   uint32_t const w = __float_as_uint(b.w);
   uint32_t const slot = w & 0x7fffffffu;
@@ -633,15 +639,12 @@ __global__ void __launch_bounds__(kBlock) k_resolve_frames(color_args a, float4 
 void free_ray_buffers(render_state& R) {
   for (void* p : {static_cast<void*>(R.gen[0]), static_cast<void*>(R.gen[1]), static_cast<void*>(R.trace),
            static_cast<void*>(R.counts), static_cast<void*>(R.block_sums), static_cast<void*>(R.fcol),
-           static_cast<void*>(R.okeys[0]), static_cast<void*>(R.okeys[1]), static_cast<void*>(R.ovals[0]),
-           static_cast<void*>(R.ovals[1]), R.otemp, static_cast<void*>(R.shadow_q)})
+           static_cast<void*>(R.shadow_q)})
     cudaFree(p);
+  free_ray_order(R.order);
   R.gen[0] = R.gen[1] = nullptr;
   R.trace = R.fcol = nullptr;
   R.counts = R.block_sums = nullptr;
-  R.okeys[0] = R.okeys[1] = R.ovals[0] = R.ovals[1] = nullptr;
-  R.otemp = nullptr;
-  R.otemp_bytes = 0;
   R.shadow_q = nullptr;
   R.frames_cap = 0;
 }
@@ -666,16 +669,6 @@ int ensure_render_buffers(myrt_ctx* ctx, uint32_t W, uint32_t H, uint32_t frames
   alloc(reinterpret_cast<void**>(&R.shadow_q), n * 32, "shadow rays");
   alloc(reinterpret_cast<void**>(&R.block_sums), std::max<size_t>(nb, 1) * sizeof(uint32_t), "block sums");
   if (frames > 1) alloc(reinterpret_cast<void**>(&R.fcol), n * 16, "frame colours");
-  // visiting order of the trace passes: one key and slot per thread of a pass's grid
-  size_t const threads = nb * kBlock;
-  for (int k = 0; k < 2; ++k) {
-    alloc(reinterpret_cast<void**>(&R.okeys[k]), threads * 4, "pass order keys");
-    alloc(reinterpret_cast<void**>(&R.ovals[k]), threads * 4, "pass order slots");
-  }
-  if (!rc)
-    rc = check_cuda(ctx, cub::DeviceRadixSort::SortPairs(nullptr, R.otemp_bytes, R.okeys[0], R.okeys[1], R.ovals[0],
-                             R.ovals[1], int(threads), 0, kOrderKeyBits, ctx->stream), "pass order size");
-  alloc(&R.otemp, std::max<size_t>(R.otemp_bytes, 16), "pass order temporary");
   if (rc) {
     free_ray_buffers(R);
     return rc;
@@ -819,16 +812,20 @@ int render_reference_frames(myrt_ctx* ctx, myrt_camera const* cam, myrt_render_p
   color_args ca = fs.ca;
   cudaStream_t const st = ctx->stream;
   uint32_t* const cnt[2] = {R.counts, R.counts + kMaxFramesInFlight};
-  // Visiting order of the trace passes (trace_order): sorted by origin / direction cell for the first
-  // two passes, which hold most of the rays, once the frames in flight fill 1 Mi slots (0); never
-  // (1); every pass (2). Results never depend on it.
+  // Visiting order (trace_order) by origin / direction cell, once the frames in flight fill 1 Mi
+  // slots, of the first two bounces' rays and of the first two passes' shadow rays, which are most of
+  // those that scattered (0); never (1); every pass (2). Results never depend on it. 64 frames of
+  // 512x512: no shadow rays 20.03, the first pass's 19.63, two 19.54, three 19.67 ms.
   uint32_t const order = ctx->tuning.trace_order;
   // NEE shadow rays of mesh-only scenes walk in their own pass, every lane with a ray (a queue
   // entry names its slot in 31 bits)
   bool const split_shadow = sd.sdf.n_drawables == 0 && size_t(K) * n < (size_t(1) << 31);
   uint32_t* const shadow_count = R.counts + 2 * kMaxFramesInFlight;
-  float3 klo, ksc;
-  ray_key_grid(ctx->scene.bounds, klo, ksc);
+  uint64_t const max_threads = uint64_t(K) * nb * kBlock;  // a slot per thread of a pass's grid
+  bool const can_sort = (order == 2 || (order == 0 && size_t(K) * n >= kOrderMin)) &&
+      ensure_ray_order(R.order, size_t(max_threads), ctx->stream);
+  pass_cell cell{nullptr, nullptr, uint32_t(n), nb, {}, {}};
+  ray_cell_grid(ctx->scene.bounds, cell.lo, cell.scale);
   for (int f0 = 0; f0 < F; f0 += int(K)) {
     uint32_t const k = std::min<uint32_t>(K, uint32_t(F - f0));
     auto rand_of = [&](int pass) {
@@ -846,25 +843,30 @@ int render_reference_frames(myrt_ctx* ctx, myrt_camera const* cam, myrt_render_p
     int pass = 1;
     for (int i = 0; i <= B; ++i) {
       bool const last = i == B;
-      bool const sorted = order == 2 || (order == 0 && i < 2 && size_t(k) * n >= (size_t(1) << 20));
-      uint32_t const* perm = nullptr;
+      bool const sorted = can_sort && (order == 2 || (i >= 1 && i <= 2 && size_t(k) * n >= kOrderMin));
       if (sorted) {
-        k_gen_keys<<<grid, kBlock, 0, st>>>(R.gen[cur], cnt[cur], uint32_t(n), nb, klo, ksc, R.okeys[0], R.ovals[0]);
-        size_t tb = R.otemp_bytes;
-        rc = check_cuda(ctx, cub::DeviceRadixSort::SortPairs(R.otemp, tb, R.okeys[0], R.okeys[1], R.ovals[0],
-                                 R.ovals[1], int(size_t(grid) * kBlock), 0, kOrderKeyBits, st), "pass order sort");
+        cell.gen = R.gen[cur];
+        cell.count = cnt[cur];
+        rc = check_cuda(ctx, build_ray_order(R.order, cell, grid * kBlock, nullptr, st), "pass order");
         if (rc) return rc;
-        perm = R.ovals[1];
       }
+      uint32_t const* const perm = sorted ? R.order.dev.perm : nullptr;
       if (split_shadow) {
         rc = check_cuda(ctx, cudaMemsetAsync(shadow_count, 0, sizeof(uint32_t), st), "shadow queue reset");
         if (rc) return rc;
       }
       k_trace_pass<<<grid, kBlock, 0, st>>>(sd, rand_of(pass), R.gen[cur], R.trace, cnt[cur], uint32_t(n), nb, perm,
           split_shadow ? R.shadow_q : nullptr, shadow_count);
-      if (split_shadow)
+      if (split_shadow) {
+        bool const sorted_shadow = can_sort && (order == 2 || (i <= 1 && size_t(k) * n >= kOrderMin));
+        if (sorted_shadow) {
+          rc = check_cuda(ctx, build_ray_order(R.order, shadow_cell{R.shadow_q, cell.lo, cell.scale},
+                                   uint32_t(size_t(k) * n), shadow_count, st), "shadow order");
+          if (rc) return rc;
+        }
         k_shadow_pass<<<uint32_t((size_t(k) * n + kShadowBlock - 1) / kShadowBlock), kShadowBlock, 0, st>>>(sd,
-            R.shadow_q, shadow_count, R.trace);
+            R.shadow_q, shadow_count, R.trace, sorted_shadow ? R.order.dev.perm : nullptr);
+      }
       ++pass;
       ca.force = last ? 1 : 0;
       k_color_pass<<<grid, kBlock, 0, st>>>(ca, rand_of(pass), R.gen[cur], R.trace, cnt[cur], R.block_sums, fcol,
