@@ -222,12 +222,13 @@ struct shadow_cell {
 // results as the reference's order.
 // gen / trace: the frames' regions of `slots` rays; count[f]: frame f's rays.
 // perm (may be null): thread t takes the ray slot of thread perm[t] of the grid.
-// shadow_q (may be null): without SDF drawables, the NEE shadow rays are
-// appended there (2 float4 each, *shadow_count of them) for k_shadow_pass
-// instead of being walked here.
-// Four resident blocks per SM (64 registers; the unbounded build used 80 and spilled as much): with
-// frames in flight the pass is issue-bound, and the extra warps measured 12 % faster together with
-// the same cap on k_color_pass (0.373 -> 0.330 ms per 512x512 frame).
+// QUEUE (scenes without SDF drawables): the NEE shadow rays are appended to
+// shadow_q (2 float4 each, *shadow_count of them) for k_shadow_pass instead of
+// being walked here.
+// Four resident blocks per SM (64 registers). The marches and the second walk are compiled in only
+// where they run: one kernel for all spilled 312 bytes under that cap, the queueing one spills 60
+// (64 frames of 512x512: 19.57 -> 19.13 ms; five blocks 19.40).
+template <bool SDF, bool QUEUE>
 __global__ void __launch_bounds__(kBlock, 4) k_trace_pass(scene_dev s, pass_rand pr, float4 const* __restrict__ gen,
     float4* __restrict__ trace, uint32_t const* __restrict__ count, uint32_t slots, uint32_t nb,
     uint32_t const* __restrict__ perm, float4* __restrict__ shadow_q, uint32_t* __restrict__ shadow_count) {
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_pass(scene_dev s, pass_rand
 
   // SDF drawables after the meshes (pt_trace.comp:342-352): a closer march hit
   // replaces the mesh hit and its attributes.
-  for (int dsdf = 0; dsdf < s.sdf.n_drawables; ++dsdf) {
+  for (int dsdf = 0; SDF && dsdf < s.sdf.n_drawables; ++dsdf) {
     sdfk::sdf_hit const sh =
         sdfk::march(s.sdf, dsdf, ro, rd, hits ? ht : __int_as_float(0x7f800000), false, &r);
     if (sh.hits && sh.t < ht) {
@@ -349,7 +350,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_pass(scene_dev s, pass_rand
   t[2] = make_float4(uv.x, uv.y, __int_as_float(material), __uint_as_float(light_color));
   t[3] = make_float4(light_dir.x, light_dir.y, light_dir.z, light_strength);
   if (!shadow) return;
-  if (shadow_q && s.sdf.n_drawables == 0) {
+  if (QUEUE) {
     // one atomic per group of converged lanes; entry: (so, dist_l), (dir_l, slot | light << 31)
     uint32_t const lanes = __activemask();
     uint32_t const lane = threadIdx.x & 31u;
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_pass(scene_dev s, pass_rand
   bool occluded = traverse<0, true, false>(s.nodes, s.tris, f3{so.x, so.y, so.z}, f3{dir_l.x, dir_l.y, dir_l.z},
       0.f, dist_l, hs, s.err, cn, ct);
   // any_hit's SDF loop (pt_trace.comp:319-327)
-  for (int dsdf = 0; !occluded && dsdf < s.sdf.n_drawables; ++dsdf)
+  for (int dsdf = 0; SDF && !occluded && dsdf < s.sdf.n_drawables; ++dsdf)
     occluded = sdfk::march(s.sdf, dsdf, so, dir_l, dist_l, true, &r).hits;
   if (occluded) return;
   v3 const col{c_lights[li].cx, c_lights[li].cy, c_lights[li].cz};
@@ -377,6 +378,11 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_pass(scene_dev s, pass_rand
   light_strength = light_strength * (2.f / dist_l);
   reinterpret_cast<float*>(t + 2)[3] = __uint_as_float(light_color);
   t[3] = make_float4(dir_l.x, dir_l.y, dir_l.z, light_strength);
+}
+
+// queue: leave the shadow rays to k_shadow_pass (meshes only)
+auto* trace_pass_of(bool sdf, bool queue) {
+  return sdf ? k_trace_pass<true, false> : queue ? k_trace_pass<false, true> : k_trace_pass<false, false>;
 }
 
 // The NEE shadow rays k_trace_pass queued (meshes only): any_hit
@@ -821,6 +827,7 @@ int render_reference_frames(myrt_ctx* ctx, myrt_camera const* cam, myrt_render_p
   // entry names its slot in 31 bits)
   bool const split_shadow = sd.sdf.n_drawables == 0 && size_t(K) * n < (size_t(1) << 31);
   uint32_t* const shadow_count = R.counts + 2 * kMaxFramesInFlight;
+  auto* const trace_pass = trace_pass_of(sd.sdf.n_drawables > 0, split_shadow);
   uint64_t const max_threads = uint64_t(K) * nb * kBlock;  // a slot per thread of a pass's grid
   bool const can_sort = (order == 2 || (order == 0 && size_t(K) * n >= kOrderMin)) &&
       ensure_ray_order(R.order, size_t(max_threads), ctx->stream);
@@ -855,8 +862,8 @@ int render_reference_frames(myrt_ctx* ctx, myrt_camera const* cam, myrt_render_p
         rc = check_cuda(ctx, cudaMemsetAsync(shadow_count, 0, sizeof(uint32_t), st), "shadow queue reset");
         if (rc) return rc;
       }
-      k_trace_pass<<<grid, kBlock, 0, st>>>(sd, rand_of(pass), R.gen[cur], R.trace, cnt[cur], uint32_t(n), nb, perm,
-          split_shadow ? R.shadow_q : nullptr, shadow_count);
+      trace_pass<<<grid, kBlock, 0, st>>>(sd, rand_of(pass), R.gen[cur], R.trace, cnt[cur], uint32_t(n), nb, perm,
+          R.shadow_q, shadow_count);
       if (split_shadow) {
         bool const sorted_shadow = can_sort && (order == 2 || (i <= 1 && size_t(k) * n >= kOrderMin));
         if (sorted_shadow) {
@@ -1003,6 +1010,7 @@ int render_reference_frames_noalloc(myrt_ctx* ctx, myrt_camera const* cam, myrt_
   color_args ca = fs.ca;
   size_t const n = size_t(W) * H;
   uint32_t const nb = uint32_t((n + kBlock - 1) / kBlock);
+  auto* const trace_pass = trace_pass_of(sd.sdf.n_drawables > 0, false);
   for (int f = 0; f < F; ++f) {  // one frame at a time: one region of ray slots
     auto rand_of = [&](int pass) {
       pass_rand pr{};
@@ -1017,7 +1025,7 @@ int render_reference_frames_noalloc(myrt_ctx* ctx, myrt_camera const* cam, myrt_
     int pass = 1;
     for (int i = 0; i <= B; ++i) {
       bool const last = i == B;
-      k_trace_pass<<<nb, kBlock, 0, st>>>(sd, rand_of(pass), gen[cur], trace, counts + cur, uint32_t(n), nb,
+      trace_pass<<<nb, kBlock, 0, st>>>(sd, rand_of(pass), gen[cur], trace, counts + cur, uint32_t(n), nb,
           nullptr, nullptr, nullptr);
       ++pass;
       ca.force = last ? 1 : 0;
