@@ -178,6 +178,7 @@ struct myrt_ctx {
   // staging buffers of the host-memory entry points (one chunk slot per lane)
   void* stage[4] = {nullptr, nullptr, nullptr, nullptr};
   size_t stage_bytes = 0;
+  void* small_stage = nullptr;   // mapped host memory of the small host queries (kSmallRays rays)
   // ray-order scratch per stream lane; `done` orders reuse across streams
   struct order_scratch {
     myrt_b200::ray_order order;
