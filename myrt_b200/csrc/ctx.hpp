@@ -144,7 +144,9 @@ struct physical_state {
   float4* hits = nullptr;               // 3 float4 per queue slot: (p, kind), (ns, t), (ng, -)
   float4* shadow = nullptr;             // 3 float4 per shadow ray: (o, path), (d, tmax), (contribution, -)
   float4* radiance = nullptr;           // per path: rgb
-  uint32_t* counts = nullptr;           // [0..1] ray queues, [2] shadow queue
+  uint32_t* counts = nullptr;           // [0..1] ray queues, [2..3] shadow queue of even / odd vertices
+  cudaStream_t side = nullptr;          // shadow rays of a vertex beside the next vertex's extension
+  cudaEvent_t shaded = nullptr, shadowed = nullptr;
   ray_order order;                      // visiting order of an extension queue
   unsigned long long* stats = nullptr;  // paths, extension rays, shadow rays (cumulative)
   void* lights = nullptr;               // ps::area_light[n_lights]

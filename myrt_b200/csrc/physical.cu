@@ -503,6 +503,14 @@ int ensure_queues(myrt_ctx* ctx, physical_state& P, size_t paths) {
   // without room for the visiting order the queues are visited as they are
   uint32_t const order = ctx->tuning.trace_order;
   if (order == 2 || (order == 0 && paths >= kOrderMin)) ensure_ray_order(P.order, paths, ctx->stream);
+  if (!P.shadowed) {
+    int rc = MYRT_OK;
+    if (!P.side) rc = check_cuda(ctx, cudaStreamCreateWithFlags(&P.side, cudaStreamNonBlocking), "shadow stream");
+    if (!rc && !P.shaded)
+      rc = check_cuda(ctx, cudaEventCreateWithFlags(&P.shaded, cudaEventDisableTiming), "shadow stream");
+    if (!rc) rc = check_cuda(ctx, cudaEventCreateWithFlags(&P.shadowed, cudaEventDisableTiming), "shadow stream");
+    if (rc) return rc;
+  }
   if (P.capacity >= paths && P.queue[0]) return MYRT_OK;
   for (void* p : {static_cast<void*>(P.queue[0]), static_cast<void*>(P.queue[1]), static_cast<void*>(P.hits),
            static_cast<void*>(P.shadow), static_cast<void*>(P.radiance), static_cast<void*>(P.counts)})
@@ -639,6 +647,12 @@ int launch_plan(myrt_ctx* ctx, physical_state& P, cudaStream_t st, pt_scene cons
   uint32_t const bps = ctx->tuning.pt_blocks_per_sm ? ctx->tuning.pt_blocks_per_sm : 8u;
   uint32_t const grid = uint32_t(std::max(ctx->sm_count, 1)) * bps;
   size_t const nj = plan.empty() ? 0 : plan[0].jobs.size();
+  bool pending = false;  // shadow rays in flight on the side stream
+  auto join = [&]() -> int {
+    if (!pending) return MYRT_OK;
+    pending = false;
+    return check_cuda(ctx, cudaStreamWaitEvent(st, P.shadowed, 0), "shadow join");
+  };
   for (size_t wi = 0; wi < plan.size(); ++wi) {
     wave_plan const& wp = plan[wi];
     pt_wave w{d_scenes, d_jobs + wi * nj, int(nj), wp.n_paths, ctx->d_err};
@@ -668,15 +682,16 @@ int launch_plan(myrt_ctx* ctx, physical_state& P, cudaStream_t st, pt_scene cons
         if (rc) return rc;
       }
       uint32_t const* const perm = sorted ? P.order.dev.perm : nullptr;
+      uint32_t* const n_shadow = P.counts + 2 + (v & 1);
       if (any_sdf)
         k_pt_extend<true><<<qgrid, kPtBlock, 0, st>>>(w, v, P.queue[cur], P.counts + cur, P.hits,
-            P.counts + (1 - cur), P.counts + 2, P.stats, perm);
+            P.counts + (1 - cur), n_shadow, P.stats, perm);
       else if (cap10)
         k_pt_extend<false, 10><<<qgrid, kPtBlock, 0, st>>>(w, v, P.queue[cur], P.counts + cur, P.hits,
-            P.counts + (1 - cur), P.counts + 2, P.stats, perm);
+            P.counts + (1 - cur), n_shadow, P.stats, perm);
       else
         k_pt_extend<false><<<qgrid, kPtBlock, 0, st>>>(w, v, P.queue[cur], P.counts + cur, P.hits,
-            P.counts + (1 - cur), P.counts + 2, P.stats, perm);
+            P.counts + (1 - cur), n_shadow, P.stats, perm);
       guide_dev gv = gd ? *gd : guide_dev{};
       if (last) gv.n_lobes = 0;
       if (gv.n_lobes > 0) {
@@ -685,15 +700,26 @@ int launch_plan(myrt_ctx* ctx, physical_state& P, cudaStream_t st, pt_scene cons
       }
       // shading in the same order appends the next queue and the shadow rays in that order too
       shade_io io{P.queue[cur], P.hits, P.counts + cur, P.queue[1 - cur], P.counts + (1 - cur), P.shadow,
-          P.counts + 2, P.radiance, gv, perm};
+          n_shadow, P.radiance, gv, perm};
+      int rc = join();
+      if (rc) return rc;
       k_pt_shade<<<qgrid, kPtBlock, 0, st>>>(w, v, io);
       if (!last && n_lights_max > 0) {
-        if (any_sdf) k_pt_shadow<true><<<qgrid, kPtBlock, 0, st>>>(w, v, P.shadow, P.counts + 2, P.radiance, P.stats);
-        else if (cap10) k_pt_shadow<false, 10><<<qgrid, kPtBlock, 0, st>>>(w, v, P.shadow, P.counts + 2, P.radiance, P.stats);
-        else k_pt_shadow<false><<<qgrid, kPtBlock, 0, st>>>(w, v, P.shadow, P.counts + 2, P.radiance, P.stats);
+        // The shadow rays and the next vertex's extension touch nothing of one another's (the paths'
+        // radiance is theirs until the next shading), so they run side by side: each launch ends with
+        // its longest walks or marches, which would leave the device idle.
+        rc = check_cuda(ctx, cudaEventRecord(P.shaded, st), "shadow fork");
+        if (!rc) rc = check_cuda(ctx, cudaStreamWaitEvent(P.side, P.shaded, 0), "shadow fork");
+        if (rc) return rc;
+        auto* const shadow = any_sdf ? k_pt_shadow<true> : cap10 ? k_pt_shadow<false, 10> : k_pt_shadow<false>;
+        shadow<<<qgrid, kPtBlock, 0, P.side>>>(w, v, P.shadow, n_shadow, P.radiance, P.stats);
+        rc = check_cuda(ctx, cudaEventRecord(P.shadowed, P.side), "shadow fork");
+        if (rc) return rc;
+        pending = true;
       }
       cur = 1 - cur;
     }
+    if (int const rc = join()) return rc;
     for (size_t j = 0; j < nj; ++j) {
       if (wp.jobs[j].rows == 0) continue;
       uint32_t const rb = (wp.jobs[j].WH + 255) / 256;
@@ -727,6 +753,9 @@ void free_physical(physical_state& P) {
            static_cast<void*>(P.stats), P.tables})
     cudaFree(p);
   free_ray_order(P.order);
+  if (P.side) cudaStreamDestroy(P.side);
+  if (P.shaded) cudaEventDestroy(P.shaded);
+  if (P.shadowed) cudaEventDestroy(P.shadowed);
   P = physical_state{};
 }
 
