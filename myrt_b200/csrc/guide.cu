@@ -62,7 +62,7 @@ struct guide_state {
   float* sums = nullptr;         // [0] loss sum, [1] weight sum
   uint32_t* counters = nullptr;  // [0] training samples collected
   float4* points = nullptr;      // 3 float4 per row
-  float4* lobes = nullptr;       // 16 float4 per row
+  float4* lobes = nullptr;       // 16 float4 per row, in tiles
   size_t rows_cap = 0;
   float4* records = nullptr;
   size_t records_cap = 0;        // in records
@@ -109,11 +109,12 @@ constexpr float kKappaMin = 0.01f, kKappaMax = 1000.f;
 // kappa / (2 pi (1 - exp(-2 kappa)))
 __device__ __forceinline__ float vmf_norm(float k) { return k / (-6.28318530717958648f * expm1f(-2.f * k)); }
 
-// ---- k_guide_gather: queue slots -> points ---------------------------------------------
+// ---- k_guide_gather: queue slots -> points, in the wave's visiting order (perm) ---------
 __global__ void __launch_bounds__(256) k_guide_gather(float4 const* __restrict__ queue, float4 const* __restrict__ hits,
-    uint32_t const* __restrict__ count, float4* __restrict__ points) {
+    uint32_t const* __restrict__ count, uint32_t const* __restrict__ perm, float4* __restrict__ points) {
   uint32_t const n = *count;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (uint32_t at = blockIdx.x * blockDim.x + threadIdx.x; at < n; at += gridDim.x * blockDim.x) {
+    uint32_t const i = perm ? __ldg(perm + at) : at;
     float4 const h0 = hits[3 * size_t(i)], h1 = hits[3 * size_t(i) + 1], h2 = hits[3 * size_t(i) + 2];
     float4 const d = queue[3 * size_t(i) + 1];
     float wo[3] = {-d.x, -d.y, -d.z};
@@ -123,9 +124,9 @@ __global__ void __launch_bounds__(256) k_guide_gather(float4 const* __restrict__
     if ((ns[0] * ng[0] + ns[1] * ng[1]) + ns[2] * ng[2] < 0.f) ns[0] = -ns[0], ns[1] = -ns[1], ns[2] = -ns[2];
     if (!((ns[0] * wo[0] + ns[1] * wo[1]) + ns[2] * wo[2] > 0.f)) ns[0] = ng[0], ns[1] = ng[1], ns[2] = ng[2];
     float const valid = __float_as_int(h0.w) >= 0 ? 1.f : 0.f;
-    points[3 * size_t(i)] = make_float4(h0.x, h0.y, h0.z, valid);
-    points[3 * size_t(i) + 1] = make_float4(ns[0], ns[1], ns[2], 0.f);
-    points[3 * size_t(i) + 2] = make_float4(wo[0], wo[1], wo[2], 0.f);
+    points[3 * size_t(at)] = make_float4(h0.x, h0.y, h0.z, valid);
+    points[3 * size_t(at) + 1] = make_float4(ns[0], ns[1], ns[2], 0.f);
+    points[3 * size_t(at) + 2] = make_float4(wo[0], wo[1], wo[2], 0.f);
   }
 }
 
@@ -284,10 +285,19 @@ __device__ __forceinline__ void second_to_stage(uint32_t tacc, uint8_t* st, uint
         make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
 }
 
-// The group's staged 128 x 128-byte tile -> half `half` of the output rows
-// (rows of 256 bytes); each warp store covers four whole 128-byte segments.
+// The group's staged 128 x 128-byte tile -> half `half` of the output rows: in
+// tiles (guide_lobes) for the shading pass, else rows of 256 bytes; each warp
+// store covers four whole 128-byte segments.
 __device__ __forceinline__ void stage_out(uint8_t const* st, uint32_t tid, uint32_t first_row, uint32_t n, int half,
-    float4* lobes) {
+    bool tiled, float4* lobes) {
+  if (tiled) {
+    if (first_row + tid >= n) return;
+    lobes += size_t(first_row >> 7) * kGuideTile + uint32_t(half) * kGuideLobes * 128u + tid;
+#pragma unroll
+    for (uint32_t c = 0; c < kGuideLobes; ++c)
+      lobes[128 * c] = *reinterpret_cast<float4 const*>(st + tc::sw128_offset(tid, c));
+    return;
+  }
 #pragma unroll
   for (uint32_t i = 0; i < 8; ++i) {
     uint32_t const idx = tid + 128u * i;
@@ -299,7 +309,7 @@ __device__ __forceinline__ void stage_out(uint8_t const* st, uint32_t tid, uint3
 }
 
 __global__ void __launch_bounds__(128 * kFwdGroups, 2) k_guide_forward(mlp_args a, float4 const* __restrict__ points,
-    uint32_t const* __restrict__ count_ptr, uint32_t n_fixed, float4* __restrict__ lobes) {
+    uint32_t const* __restrict__ count_ptr, uint32_t n_fixed, bool tiled, float4* __restrict__ lobes) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = align1024(smem_raw);
   uint8_t* wt = sm + kFwdW;
@@ -370,11 +380,11 @@ __global__ void __launch_bounds__(128 * kFwdGroups, 2) k_guide_forward(mlp_args 
       } else {
         head_to_stage(tacc, bias + 64 * l, p.w, ht, tid);
         tc::named_bar_sync(bar_id, 128);
-        stage_out(ht, tid, tile * 128u, n, 0, lobes);
+        stage_out(ht, tid, tile * 128u, n, 0, tiled, lobes);
         tc::named_bar_sync(bar_id, 128);
         second_to_stage(tacc, ht, tid);
         tc::named_bar_sync(bar_id, 128);
-        stage_out(ht, tid, tile * 128u, n, 1, lobes);
+        stage_out(ht, tid, tile * 128u, n, 1, tiled, lobes);
         tc::named_bar_sync(bar_id, 128);  // the tile is rewritten next
       }
     }
@@ -974,11 +984,11 @@ mlp_args make_mlp(myrt_ctx* ctx) {
 }
 
 int launch_forward(myrt_ctx* ctx, mlp_args const& a, float4 const* points, uint32_t const* count, uint32_t n_fixed,
-    size_t max_rows, float4* lobes, cudaStream_t st) {
+    size_t max_rows, bool tiled, float4* lobes, cudaStream_t st) {
   uint32_t const tiles = uint32_t((max_rows + 127) / 128);
   uint32_t const ctas = (tiles + kFwdGroups - 1) / kFwdGroups;
   uint32_t const grid = std::max(1u, std::min(ctas, uint32_t(std::max(ctx->sm_count, 1)) * 2u));
-  k_guide_forward<<<grid, 128 * kFwdGroups, kFwdSmem, st>>>(a, points, count, n_fixed, lobes);
+  k_guide_forward<<<grid, 128 * kFwdGroups, kFwdSmem, st>>>(a, points, count, n_fixed, tiled, lobes);
   return check_cuda(ctx, cudaGetLastError(), "guide forward launch");
 }
 
@@ -1032,7 +1042,8 @@ int guide_prepare(myrt_ctx* ctx, size_t paths, myrt_render_params const* p, guid
     g.points = g.lobes = nullptr;
     g.rows_cap = 0;
     rc = check_cuda(ctx, cudaMalloc(reinterpret_cast<void**>(&g.points), paths * 48), "guide points");
-    if (!rc) rc = check_cuda(ctx, cudaMalloc(reinterpret_cast<void**>(&g.lobes), paths * 256), "guide lobes");
+    if (!rc) rc = check_cuda(ctx, cudaMalloc(reinterpret_cast<void**>(&g.lobes), ((paths + 127) / 128) * kGuideTile * sizeof(float4)),
+                      "guide lobes");
     if (rc) return rc;
     g.rows_cap = paths;
   }
@@ -1072,14 +1083,14 @@ void guide_begin_wave(myrt_ctx* ctx, guide_dev& gd) {
 }
 
 int guide_infer(myrt_ctx* ctx, guide_dev const& gd, uint32_t, uint32_t, float4 const* queue, float4 const* hits,
-    uint32_t const* count, cudaStream_t st) {
+    uint32_t const* count, uint32_t const* perm, cudaStream_t st) {
   if (gd.n_lobes == 0) return MYRT_OK;
   guide_state& g = *ctx->guide;
   uint32_t const grid = uint32_t(std::max(ctx->sm_count, 1)) * 4u;
-  k_guide_gather<<<grid, 256, 0, st>>>(queue, hits, count, g.points);
+  k_guide_gather<<<grid, 256, 0, st>>>(queue, hits, count, perm, g.points);
   int rc = check_cuda(ctx, cudaGetLastError(), "guide gather launch");
   if (rc) return rc;
-  return launch_forward(ctx, make_mlp(ctx), g.points, count, 0, gd.paths, g.lobes, st);
+  return launch_forward(ctx, make_mlp(ctx), g.points, count, 0, gd.paths, true, g.lobes, st);
 }
 
 int guide_train(myrt_ctx* ctx, guide_dev const& gd, uint32_t paths, int max_depth, float4 const* radiance,
@@ -1165,7 +1176,7 @@ int guide_eval(myrt_ctx* ctx, float const* points, uint32_t n, float* lobes) {
   auto* const d_lobes = static_cast<float4*>(g.call_buf);
   auto* const d_pts = d_lobes + size_t(n) * 16;
   rc = check_cuda(ctx, cudaMemcpyAsync(d_pts, points, size_t(n) * 48, cudaMemcpyHostToDevice, st), "upload");
-  if (!rc) rc = launch_forward(ctx, make_mlp(ctx), d_pts, nullptr, n, n, d_lobes, st);
+  if (!rc) rc = launch_forward(ctx, make_mlp(ctx), d_pts, nullptr, n, n, false, d_lobes, st);
   if (!rc) rc = check_cuda(ctx, cudaMemcpyAsync(lobes, d_lobes, size_t(n) * 256, cudaMemcpyDeviceToHost, st), "read");
   if (!rc) rc = check_cuda(ctx, cudaStreamSynchronize(st), "guide eval");
   call_release(g);

@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(kPtBlock, 6) k_pt_shade(pt_wave w, int v, shad
           v3 const org = pos + ng * kOffset;
           guide_lobes gl;
           bool const gwave = io.guide.n_lobes > 0;
-          bool const guided = gwave && guide_load(io.guide, i, gl) && io.guide.fraction > 0.f;
+          bool const guided = gwave && guide_load(io.guide, i0, gl) && io.guide.fraction > 0.f;
           // next-event estimation
           if (s.n_lights > 0) {
             int l = 0;
@@ -695,7 +695,7 @@ int launch_plan(myrt_ctx* ctx, physical_state& P, cudaStream_t st, pt_scene cons
       guide_dev gv = gd ? *gd : guide_dev{};
       if (last) gv.n_lobes = 0;
       if (gv.n_lobes > 0) {
-        int rc = guide_infer(ctx, gv, 0, 0, P.queue[cur], P.hits, P.counts + cur, st);
+        int rc = guide_infer(ctx, gv, 0, 0, P.queue[cur], P.hits, P.counts + cur, perm, st);
         if (rc) return rc;
       }
       // shading in the same order appends the next queue and the shadow rays in that order too
