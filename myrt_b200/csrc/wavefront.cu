@@ -56,7 +56,8 @@ namespace {
 using rs::v2;
 using rs::v3;
 
-constexpr int kBlock = 256;
+constexpr int kBlock = 256;      // ray slots per block sum of the compaction
+constexpr int kWalkBlock = 128;  // threads per block of the trace and colour passes
 constexpr int kTexSize = 1024;
 constexpr int kMaxFramesInFlight = 64;
 
@@ -73,6 +74,10 @@ struct pass_rand {
 struct frame_slot {
   uint32_t f, id;
 };
+__device__ __forceinline__ frame_slot slot_of(uint32_t thread, uint32_t nb) {  // thread of a pass's grid
+  uint32_t const f = thread / (nb * kBlock);
+  return {f, thread - f * nb * kBlock};
+}
 __device__ __forceinline__ frame_slot frame_of(uint32_t nb) {
   uint32_t const f = blockIdx.x / nb;
   return {f, (blockIdx.x - f * nb) * blockDim.x + threadIdx.x};
@@ -225,18 +230,17 @@ struct shadow_cell {
 // QUEUE (scenes without SDF drawables): the NEE shadow rays are appended to
 // shadow_q (2 float4 each, *shadow_count of them) for k_shadow_pass instead of
 // being walked here.
-// Four resident blocks per SM (64 registers). The marches and the second walk are compiled in only
+// Eight resident blocks per SM (64 registers): a block keeps its registers until its longest walk
+// ends, and blocks of 256 threads measured 19.13 ms where these take 18.66 (64 threads 19.67). The marches and the second walk are compiled in only
 // where they run: one kernel for all spilled 312 bytes under that cap, the queueing one spills 60
 // (64 frames of 512x512: 19.57 -> 19.13 ms; five blocks 19.40).
 template <bool SDF, bool QUEUE>
-__global__ void __launch_bounds__(kBlock, 4) k_trace_pass(scene_dev s, pass_rand pr, float4 const* __restrict__ gen,
+__global__ void __launch_bounds__(kWalkBlock, 8) k_trace_pass(scene_dev s, pass_rand pr, float4 const* __restrict__ gen,
     float4* __restrict__ trace, uint32_t const* __restrict__ count, uint32_t slots, uint32_t nb,
     uint32_t const* __restrict__ perm, float4* __restrict__ shadow_q, uint32_t* __restrict__ shadow_count) {
   uint32_t thread = blockIdx.x * blockDim.x + threadIdx.x;
   if (perm) thread = __ldg(perm + thread);
-  frame_slot fs;
-  fs.f = thread / (nb * kBlock);
-  fs.id = thread - fs.f * nb * kBlock;
+  frame_slot const fs = slot_of(thread, nb);
   uint32_t const id = fs.id;
   if (id >= count[fs.f]) return;
   float const* const tex = pr.tex + fs.f * pr.tex_stride;
@@ -862,7 +866,7 @@ int render_reference_frames(myrt_ctx* ctx, myrt_camera const* cam, myrt_render_p
         rc = check_cuda(ctx, cudaMemsetAsync(shadow_count, 0, sizeof(uint32_t), st), "shadow queue reset");
         if (rc) return rc;
       }
-      trace_pass<<<grid, kBlock, 0, st>>>(sd, rand_of(pass), R.gen[cur], R.trace, cnt[cur], uint32_t(n), nb, perm,
+      trace_pass<<<grid * (kBlock / kWalkBlock), kWalkBlock, 0, st>>>(sd, rand_of(pass), R.gen[cur], R.trace, cnt[cur], uint32_t(n), nb, perm,
           R.shadow_q, shadow_count);
       if (split_shadow) {
         bool const sorted_shadow = can_sort && (order == 2 || (i <= 1 && size_t(k) * n >= kOrderMin));
@@ -1025,7 +1029,7 @@ int render_reference_frames_noalloc(myrt_ctx* ctx, myrt_camera const* cam, myrt_
     int pass = 1;
     for (int i = 0; i <= B; ++i) {
       bool const last = i == B;
-      trace_pass<<<nb, kBlock, 0, st>>>(sd, rand_of(pass), gen[cur], trace, counts + cur, uint32_t(n), nb,
+      trace_pass<<<nb * (kBlock / kWalkBlock), kWalkBlock, 0, st>>>(sd, rand_of(pass), gen[cur], trace, counts + cur, uint32_t(n), nb,
           nullptr, nullptr, nullptr);
       ++pass;
       ca.force = last ? 1 : 0;
