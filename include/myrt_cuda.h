@@ -193,9 +193,10 @@ typedef struct myrt_tuning {
                                 baked tree. */
   uint32_t pt_grid;          /* physical / guided extend, shade and shadow kernels: 0 = default (2),
                                 1 = grid-stride loops over pt_blocks_per_sm resident blocks per SM,
-                                2 = one thread per queue entry (the grid covers the wave's paths;
-                                blocks past the queue's count return at once; the mesh traversal
-                                kernels run at 64 registers, or under a 48-register cap when
+                                2 = one thread per queue entry (the grid covers the wave's paths
+                                up to 16 times the blocks the device holds, which then walk over
+                                the rest; the mesh traversal kernels run at 64 registers, or under a
+                                48-register cap when
                                 pt_blocks_per_sm is 10 or more).
                                 Results never depend on it. */
   uint32_t ref_frames;       /* reference shading (myrt_render): frames of one call whose passes run
@@ -221,7 +222,7 @@ int myrt_get_tuning(myrt_ctx* ctx, myrt_tuning* tuning);
 
 /* Device-time accounting of the closest / any-hit queries (no counterpart in
  * the reference): while enabled, each query records CUDA events around its
- * ordering phase (ray keys + radix sort) and its traversal kernel.
+ * ordering phase (the visiting order) and its traversal kernel.
  * myrt_get_phase_times waits for the recorded queries, returns the summed
  * milliseconds and the number of traversal launches since the last call, and
  * clears them: one per device-memory query, one per chunk of a host-memory

@@ -656,10 +656,14 @@ int launch_plan(myrt_ctx* ctx, physical_state& P, cudaStream_t st, pt_scene cons
   for (size_t wi = 0; wi < plan.size(); ++wi) {
     wave_plan const& wp = plan[wi];
     pt_wave w{d_scenes, d_jobs + wi * nj, int(nj), wp.n_paths, ctx->d_err};
-    // extend / shade / shadow: queue entries (at most the wave's paths) per thread
+    // extend / shade / shadow: a thread per queue entry (at most the wave's paths), but no more than 16
+    // times the blocks the device holds, which walk over the rest: the host does not know how few
+    // entries a late queue has, and a block for every 128 of 16 Mi paths took 70-90 us to come and go.
+    // 512x512, 64 spp: no cap 22.08 ms; 2, 4, 8, 16, 32 times 23.36, 21.89, 21.23, 21.11, 21.25
     bool const per_entry = ctx->tuning.pt_grid != 1;
     uint32_t const qgrid = per_entry
-        ? std::max<uint32_t>(1u, uint32_t((uint64_t(wp.n_paths) + kPtBlock - 1) / kPtBlock))
+        ? uint32_t(std::min<uint64_t>(std::max<uint64_t>(1u, (uint64_t(wp.n_paths) + kPtBlock - 1) / kPtBlock),
+              uint64_t(std::max(ctx->sm_count, 1)) * 8u * 16u))
         : grid;
     // the mesh traversal kernels at 64 registers; under a 48-register cap (pt_blocks_per_sm >= 10) they
     // spill 156 bytes: 24.3 against 23.6 ms per 512x512 64-spp frame
