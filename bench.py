@@ -12,9 +12,9 @@ Workload (one step = one closest-hit launch over one ray batch):
 Multi-GPU: one process per GPU, each tracing its own batch (weak scaling, no
 collective on the data path); time = max over ranks of the device time.
 
-Arms: default = this framework (CUDA, sm_100a); each step sorts the batch's
-visiting order by origin and direction cell (CUB radix sort of ray indices),
-then traces. `--impl reference` = the reference's CPU path (its BVH build +
+Arms: default = this framework (CUDA, sm_100a); each step orders the batch's
+rays by origin and direction cell (a counting sort of the warps whose rays lie
+in many cells), then traces. `--impl reference` = the reference's CPU path (its BVH build +
 its GLSL traversal and intersector compiled as C++, oracle/_ref) on the host
 cores, on a bounded sample of the same rays.
 """
@@ -535,7 +535,7 @@ def c1_run(local: int, args) -> dict:
                    "d2h_bytes_per_step": n * HIT_BYTES, "steps": e2e_steps,
                    "api": "myrt_trace_closest (host pinned buffers)", "roofline": e2e_pcie},
            "clocks": clocks.summary(),
-           "gpu_launches": args.steps * (1 if order == 1 else 2)}
+           "gpu_launches": args.steps * (1 if order == 1 else 4)}
     if not args.no_cpu_baseline:
         sys.path.insert(0, str(ROOT / "oracle"))
         import pyoracle as po
@@ -677,14 +677,14 @@ def run_ours(args):
                      "note": "algorithmic bytes = 80 B/node + 48 B/triangle + 48 B ray+hit; the 37 MB BVH is "
                              "L2-resident, so most node bytes are served by L2. achieved = those bytes over "
                              "k_trace's CUDA-event duration; frac_whole_step also counts the ordering phase "
-                             "(ray keys + radix sort of the visiting order)"},
+                             "(the visiting order's three kernels)"},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": n * RAY_BYTES,
                 "d2h_bytes_per_step": n * HIT_BYTES, "steps": e2e_steps,
                 "api": "myrt_trace_closest (host pinned buffers, chunked copy/compute overlap)",
                 "roofline": e2e_pcie},
         "clocks": clocks.summary(),
-        "gpu_launches": 2 * args.steps,
-        "gpu_launches_note": "per step: k_ray_keys + k_trace (ours) and the CUB radix sort of the visiting order",
+        "gpu_launches": 4 * args.steps,
+        "gpu_launches_note": "per step: k_order_cells, k_order_offsets, k_order_scatter and k_trace",
         "gpu_launches_e2e": e2e_steps * chunks,
     }
     # the same batch on a tree built on the device (linear BVH + 8-wide collapse)
@@ -976,11 +976,11 @@ def run_render_workload(args, emit: bool = True):
          "e2e": {"value": samples / e2e_s, "unit": "samples/s", "h2d_bytes_per_step": 128 + frames * passes * 4096,
                  "d2h_bytes_per_step": W * H * 16 * 2, "api": "myrt_render + myrt_read_accumulation"},
          "frames_in_flight": k_fl,
-         "gpu_launches": n_batches * (1 + 3 * (B + 1) + 2 * B + 2) + (n_batches if k_fl > 1 else 0),
+         "gpu_launches": n_batches * (1 + 3 * (B + 1) + 2 * B + 12) + (n_batches if k_fl > 1 else 0),
          "gpu_launches_note": "per batch of frames in flight: generate; per bounce trace, shadow and color, plus "
-                              "scan + scatter of the surviving rays after every bounce but the last; the visiting-"
-                              "order keys of the first two trace passes; the in-order resolve of the batch's frames "
-                              "into the accumulation (CUB's radix-sort kernels not counted)",
+                              "scan + scatter of the surviving rays after every bounce but the last; three kernels "
+                              "for the visiting order of two trace and two shadow passes; the in-order resolve of "
+                              "the batch's frames into the accumulation",
          "cpu_baseline": cpu,
          "clocks": clocks.summary()})
     if not emit:
@@ -1162,7 +1162,8 @@ def _sdf_fp32_roofline():
     peak = 148 * 128 * 2 * mhz * 1e6 / 1e12
     return {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak if achieved else None,
-            "source": "ncu FP32 thread-instruction counts of k_pt_extend<1> (one launch, 1 Mi camera rays); peak "
+            "source": "ncu FP32 thread-instruction counts of k_pt_extend<1> as an interpreter (one launch, 1 Mi "
+                      "camera rays), before left folds were compiled into records; peak "
                       "nominal at sm_max_mhz; the evaluator runs without FMA contraction (bit-exact with the "
                       "reference's march) and is bound by divergent issue, not FP32 throughput"}
 

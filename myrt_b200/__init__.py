@@ -136,7 +136,7 @@ class Context:
 
     def phase_times(self) -> dict:
         """Summed device milliseconds of the queries since the last call: order_ms
-        (ray keys + radix sort), traverse_ms (traversal kernel), queries."""
+        (the visiting order), traverse_ms (traversal kernel), queries."""
         o, t, q = C.c_double(), C.c_double(), C.c_uint64()
         self._check(self._L.myrt_get_phase_times(self._h, C.byref(o), C.byref(t), C.byref(q)),
                     "myrt_get_phase_times")

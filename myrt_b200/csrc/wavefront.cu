@@ -231,9 +231,9 @@ struct shadow_cell {
 // shadow_q (2 float4 each, *shadow_count of them) for k_shadow_pass instead of
 // being walked here.
 // Eight resident blocks per SM (64 registers): a block keeps its registers until its longest walk
-// ends, and blocks of 256 threads measured 19.13 ms where these take 18.66 (64 threads 19.67). The marches and the second walk are compiled in only
-// where they run: one kernel for all spilled 312 bytes under that cap, the queueing one spills 60
-// (64 frames of 512x512: 19.57 -> 19.13 ms; five blocks 19.40).
+// ends, and blocks of 256 threads measured 19.13 ms where these take 18.66 (64 threads 19.67). The
+// marches and the second walk are compiled in only where they run: one kernel for all spilled 312
+// bytes under that cap, the queueing one spills 60 (64 frames of 512x512: 19.57 -> 19.13 ms).
 template <bool SDF, bool QUEUE>
 __global__ void __launch_bounds__(kWalkBlock, 8) k_trace_pass(scene_dev s, pass_rand pr, float4 const* __restrict__ gen,
     float4* __restrict__ trace, uint32_t const* __restrict__ count, uint32_t slots, uint32_t nb,
