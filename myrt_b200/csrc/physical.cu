@@ -43,6 +43,7 @@
 #include "sdf.cuh"
 #include "trace.cuh"
 #include "rayorder.cuh"
+#include "stream_fork.hpp"
 
 namespace myrt_b200 {
 
@@ -647,12 +648,7 @@ int launch_plan(myrt_ctx* ctx, physical_state& P, cudaStream_t st, pt_scene cons
   uint32_t const bps = ctx->tuning.pt_blocks_per_sm ? ctx->tuning.pt_blocks_per_sm : 8u;
   uint32_t const grid = uint32_t(std::max(ctx->sm_count, 1)) * bps;
   size_t const nj = plan.empty() ? 0 : plan[0].jobs.size();
-  bool pending = false;  // shadow rays in flight on the side stream
-  auto join = [&]() -> int {
-    if (!pending) return MYRT_OK;
-    pending = false;
-    return check_cuda(ctx, cudaStreamWaitEvent(st, P.shadowed, 0), "shadow join");
-  };
+  stream_fork side(st, P.side, P.shaded, P.shadowed);  // a vertex's shadow rays; joined on every way out
   for (size_t wi = 0; wi < plan.size(); ++wi) {
     wave_plan const& wp = plan[wi];
     pt_wave w{d_scenes, d_jobs + wi * nj, int(nj), wp.n_paths, ctx->d_err};
@@ -705,25 +701,23 @@ int launch_plan(myrt_ctx* ctx, physical_state& P, cudaStream_t st, pt_scene cons
       // shading in the same order appends the next queue and the shadow rays in that order too
       shade_io io{P.queue[cur], P.hits, P.counts + cur, P.queue[1 - cur], P.counts + (1 - cur), P.shadow,
           n_shadow, P.radiance, gv, perm};
-      int rc = join();
+      int rc = check_cuda(ctx, side.join(), "shadow join");
       if (rc) return rc;
       k_pt_shade<<<qgrid, kPtBlock, 0, st>>>(w, v, io);
       if (!last && n_lights_max > 0) {
         // The shadow rays and the next vertex's extension touch nothing of one another's (the paths'
         // radiance is theirs until the next shading), so they run side by side: each launch ends with
         // its longest walks or marches, which would leave the device idle.
-        rc = check_cuda(ctx, cudaEventRecord(P.shaded, st), "shadow fork");
-        if (!rc) rc = check_cuda(ctx, cudaStreamWaitEvent(P.side, P.shaded, 0), "shadow fork");
+        rc = check_cuda(ctx, side.fork(), "shadow fork");
         if (rc) return rc;
         auto* const shadow = any_sdf ? k_pt_shadow<true> : cap10 ? k_pt_shadow<false, 10> : k_pt_shadow<false>;
         shadow<<<qgrid, kPtBlock, 0, P.side>>>(w, v, P.shadow, n_shadow, P.radiance, P.stats);
-        rc = check_cuda(ctx, cudaEventRecord(P.shadowed, P.side), "shadow fork");
+        rc = check_cuda(ctx, side.launched(), "shadow fork");
         if (rc) return rc;
-        pending = true;
       }
       cur = 1 - cur;
     }
-    if (int const rc = join()) return rc;
+    if (int const rc = check_cuda(ctx, side.join(), "shadow join")) return rc;
     for (size_t j = 0; j < nj; ++j) {
       if (wp.jobs[j].rows == 0) continue;
       uint32_t const rb = (wp.jobs[j].WH + 255) / 256;
