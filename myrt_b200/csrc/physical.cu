@@ -501,9 +501,6 @@ void mat_mul4(float const* a, float const* b, float* out) {
 }
 
 int ensure_queues(myrt_ctx* ctx, physical_state& P, size_t paths) {
-  // without room for the visiting order the queues are visited as they are
-  uint32_t const order = ctx->tuning.trace_order;
-  if (order == 2 || (order == 0 && paths >= kOrderMin)) ensure_ray_order(P.order, paths, ctx->stream);
   if (!P.shadowed) {
     int rc = MYRT_OK;
     if (!P.side) rc = check_cuda(ctx, cudaStreamCreateWithFlags(&P.side, cudaStreamNonBlocking), "shadow stream");
@@ -519,6 +516,7 @@ int ensure_queues(myrt_ctx* ctx, physical_state& P, size_t paths) {
   P.queue[0] = P.queue[1] = P.hits = P.shadow = P.radiance = nullptr;
   P.counts = nullptr;
   P.capacity = 0;
+  if (P.order.cap < paths) free_ray_order(P.order);  // made again, where there is room, by ensure_queue_order
   int rc = MYRT_OK;
   auto alloc = [&](void** p, size_t bytes, char const* what) {
     if (!rc) rc = check_cuda(ctx, cudaMalloc(p, bytes), what);
@@ -536,6 +534,14 @@ int ensure_queues(myrt_ctx* ctx, physical_state& P, size_t paths) {
   if (rc) return rc;
   P.capacity = paths;
   return MYRT_OK;
+}
+
+// The visiting order's scratch, which a wave can do without: taken after everything it cannot do
+// without (queues, the guide's points and lobes, tables). Without room for it the queues are visited
+// as they are.
+void ensure_queue_order(myrt_ctx* ctx, physical_state& P, size_t paths) {
+  uint32_t const order = ctx->tuning.trace_order;
+  if (order == 2 || (order == 0 && paths >= kOrderMin)) ensure_ray_order(P.order, paths, ctx->stream);
 }
 
 pt_scene scene_of(myrt_ctx const* ctx) {
@@ -888,6 +894,7 @@ int render_physical_frames(myrt_ctx* ctx, myrt_camera const* cam, myrt_render_pa
   size_t const bytes = sizeof(pt_scene) + plan.size() * sizeof(pt_job);
   rc = grow_bytes(ctx, &P.tables, P.tables_cap, bytes, "wave tables");
   if (rc) return rc;
+  ensure_queue_order(ctx, P, max_paths);
   std::vector<unsigned char> host(bytes);
   std::memcpy(host.data(), &sc, sizeof(pt_scene));
   for (size_t i = 0; i < plan.size(); ++i)
@@ -963,6 +970,7 @@ int build_graph(myrt_batch* b) {
     if (rc) return rc;
     b->d_jobs_cap = bytes;
   }
+  ensure_queue_order(ctx, b->queues, max_paths);
   for (size_t w = 0; w < b->plan.size(); ++w)
     std::memcpy(b->h_jobs + w * nj, b->plan[w].jobs.data(), nj * sizeof(pt_job));
   cudaStream_t const st = ctx->stream;
