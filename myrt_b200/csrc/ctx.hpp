@@ -13,6 +13,7 @@
 #include "bvh8.hpp"
 #include "bvh8_device.hpp"
 #include "instances.hpp"
+#include "rayorder.hpp"
 
 namespace myrt_b200 {
 
@@ -96,20 +97,6 @@ struct device_sdf {
   uint2* chain_list = nullptr;
   int n_drawables = 0;
   int n_programs = 0;
-};
-
-// Scratch of a visiting order (rayorder.cuh); 12 bytes per slot and 32 MB.
-struct ray_order_dev {
-  uint32_t* count = nullptr;   // rays per cell, zero between uses
-  uint32_t* offset = nullptr;  // first position of a cell's rays
-  uint2* rec = nullptr;        // (cell, rank) of every ray of the warps taken apart
-  uint32_t* warp = nullptr;    // those warps' first slots
-  uint32_t* perm = nullptr;    // the order: slot of the i-th thread
-  uint32_t* ctr = nullptr;     // warps taken apart, rays of the others, positions given out
-};
-struct ray_order {
-  ray_order_dev dev;
-  size_t cap = 0;  // slots
 };
 
 // Wavefront render state (sequential_pathtracer's buffers and counters).

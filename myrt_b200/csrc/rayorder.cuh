@@ -27,15 +27,12 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
-#include "ctx.hpp"
+#include "rayorder.hpp"
 
 namespace myrt_b200 {
 
 // Batches from this size on are ordered (trace_order 0).
 constexpr uint32_t kOrderMin = 1u << 20;
-constexpr uint32_t kOrderCells = 1u << 22;
-constexpr uint32_t kOrderChunk = 4096;                       // cells per block of k_order_offsets
-constexpr uint32_t kOrderBins = kOrderCells + kOrderChunk;   // and the cell of empty slots
 constexpr uint32_t kOrderTile = 1024;                        // rays per block of k_order_cells
 constexpr uint32_t kOrderScatterBlocks = 148 * 8;            // one resident wave, however few warps were taken apart
 // Camera rays of a 1024 x 1024 image lie in 1.3 cells per warp, of a 512 x 512 one in 1.5, shadow
@@ -178,45 +175,15 @@ inline void ray_cell_grid(float const* b, float3& lo, float3& cell_scale) {
   }
 }
 
-inline void free_ray_order(ray_order& o) {
-  for (void* p : {static_cast<void*>(o.dev.count), static_cast<void*>(o.dev.offset), static_cast<void*>(o.dev.rec),
-           static_cast<void*>(o.dev.warp), static_cast<void*>(o.dev.perm), static_cast<void*>(o.dev.ctr)})
-    cudaFree(p);
-  o.dev = ray_order_dev{};
-  o.cap = 0;
-}
-
-// Room for n slots. False, with nothing held and no error left behind, when the
-// device has none: the caller then visits in input order.
-inline bool ensure_ray_order(ray_order& o, size_t n, cudaStream_t s) {
-  if (o.cap >= n && o.dev.perm) return true;
-  if (cudaStreamSynchronize(s) != cudaSuccess) return false;
-  free_ray_order(o);
-  auto alloc = [](auto** p, size_t bytes) { return cudaMalloc(reinterpret_cast<void**>(p), bytes) == cudaSuccess; };
-  size_t const warps = (n + 31) / 32;
-  if (alloc(&o.dev.count, size_t(kOrderBins) * 4) && alloc(&o.dev.offset, size_t(kOrderBins) * 4) &&
-      alloc(&o.dev.rec, warps * 32 * 8) && alloc(&o.dev.warp, warps * 4) && alloc(&o.dev.perm, warps * 32 * 4) &&
-      alloc(&o.dev.ctr, 4 * sizeof(uint32_t)) &&
-      cudaMemsetAsync(o.dev.count, 0, size_t(kOrderBins) * 4, s) == cudaSuccess) {
-    o.cap = n;
-    return true;
-  }
-  cudaGetLastError();
-  free_ray_order(o);
-  return false;
-}
-
 // The order of n slots into o.dev.perm (room for them made before).
 template <class CELL>
-cudaError_t build_ray_order(ray_order const& o, CELL const& cell_of, uint32_t n, uint32_t const* n_dev,
-    cudaStream_t s) {
-  cudaError_t const e = cudaMemsetAsync(o.dev.ctr, 0, 4 * sizeof(uint32_t), s);
-  if (e != cudaSuccess) return e;
-  ray_order_dev const r = o.dev;
-  k_order_cells<<<uint32_t((size_t(n) + kOrderTile - 1) / kOrderTile), 256, 0, s>>>(cell_of, n, n_dev, r);
-  k_order_offsets<<<kOrderBins / kOrderChunk, kOrderChunk / 4, 0, s>>>(r);
-  k_order_scatter<<<std::min(kOrderScatterBlocks, uint32_t((size_t(n) + 255) / 256)), 256, 0, s>>>(n, n_dev, r);
-  return cudaGetLastError();
+cudaError_t build_ray_order(ray_order& o, CELL const& cell_of, uint32_t n, uint32_t const* n_dev, cudaStream_t s) {
+  return use_ray_order(o, s, [&] {
+    ray_order_dev const r = o.dev;
+    k_order_cells<<<uint32_t((size_t(n) + kOrderTile - 1) / kOrderTile), 256, 0, s>>>(cell_of, n, n_dev, r);
+    k_order_offsets<<<kOrderBins / kOrderChunk, kOrderChunk / 4, 0, s>>>(r);
+    k_order_scatter<<<std::min(kOrderScatterBlocks, uint32_t((size_t(n) + 255) / 256)), 256, 0, s>>>(n, n_dev, r);
+  });
 }
 
 }  // namespace myrt_b200

@@ -1,0 +1,76 @@
+// Host side of a visiting order's scratch (rayorder.cuh): its arrays, and what
+// holds between uses.
+#pragma once
+#include <cstddef>
+#include <cstdint>
+#include <cuda_runtime_api.h>
+
+namespace myrt_b200 {
+
+constexpr uint32_t kOrderCells = 1u << 22;
+constexpr uint32_t kOrderChunk = 4096;                       // cells per block of k_order_offsets
+constexpr uint32_t kOrderBins = kOrderCells + kOrderChunk;   // and the cell of empty slots
+
+// 12 bytes per slot and 32 MB.
+struct ray_order_dev {
+  uint32_t* count = nullptr;   // rays per cell, zero between uses
+  uint32_t* offset = nullptr;  // first position of a cell's rays
+  uint2* rec = nullptr;        // (cell, rank) of every ray of the warps taken apart
+  uint32_t* warp = nullptr;    // those warps' first slots
+  uint32_t* perm = nullptr;    // the order: slot of the i-th thread
+  uint32_t* ctr = nullptr;     // warps taken apart, rays of the others, positions given out
+};
+struct ray_order {
+  ray_order_dev dev;
+  size_t cap = 0;      // slots
+  bool clean = false;  // the counts are zero; not after a use whose launches may have run in part
+};
+
+inline void free_ray_order(ray_order& o) {
+  for (void* p : {static_cast<void*>(o.dev.count), static_cast<void*>(o.dev.offset), static_cast<void*>(o.dev.rec),
+           static_cast<void*>(o.dev.warp), static_cast<void*>(o.dev.perm), static_cast<void*>(o.dev.ctr)})
+    cudaFree(p);
+  o = ray_order{};
+}
+
+// Room for n slots, with zero counts. False, with nothing held and no error left
+// behind, when the device has none: the caller then visits in input order.
+inline bool ensure_ray_order(ray_order& o, size_t n, cudaStream_t s) {
+  if (o.cap >= n && o.dev.perm && o.clean) return true;
+  if (cudaStreamSynchronize(s) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (o.cap < n || !o.dev.perm) {
+    free_ray_order(o);
+    auto alloc = [](auto** p, size_t bytes) { return cudaMalloc(reinterpret_cast<void**>(p), bytes) == cudaSuccess; };
+    size_t const warps = (n + 31) / 32;
+    if (alloc(&o.dev.count, size_t(kOrderBins) * 4) && alloc(&o.dev.offset, size_t(kOrderBins) * 4) &&
+        alloc(&o.dev.rec, warps * 32 * 8) && alloc(&o.dev.warp, warps * 4) && alloc(&o.dev.perm, warps * 32 * 4) &&
+        alloc(&o.dev.ctr, 4 * sizeof(uint32_t)))
+      o.cap = n;
+  }
+  if (o.cap >= n && cudaMemsetAsync(o.dev.count, 0, size_t(kOrderBins) * 4, s) == cudaSuccess) {
+    o.clean = true;
+    return true;
+  }
+  cudaGetLastError();
+  free_ray_order(o);
+  return false;
+}
+
+// One use: launch() starts the kernels that count, turn counts into positions
+// (zeroing them again) and scatter. Counts that a failed launch leaves behind
+// would push a later use's positions past the order's end, so the scratch is
+// then unfit until ensure_ray_order has cleared it.
+template <class LAUNCH>
+cudaError_t use_ray_order(ray_order& o, cudaStream_t s, LAUNCH const& launch) {
+  o.clean = false;
+  cudaError_t const e = cudaMemsetAsync(o.dev.ctr, 0, 4 * sizeof(uint32_t), s);
+  if (e == cudaSuccess) launch();
+  cudaError_t const l = cudaGetLastError();  // also takes back the clearing's own error
+  o.clean = e == cudaSuccess && l == cudaSuccess;
+  return e != cudaSuccess ? e : l;
+}
+
+}  // namespace myrt_b200

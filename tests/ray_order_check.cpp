@@ -1,0 +1,69 @@
+// Host check of rayorder.hpp over the fake runtime (fake_cuda.hpp): a sequence
+// of uses of growing size on a device with and without room, with a failure at
+// every call and at every launch. Whenever the kernels are launched, the arrays
+// hold the slots asked for and the counts are zero; a failure leaves nothing
+// that a later, sound use could trip over; freeing leaves nothing behind.
+// Prints the cases checked.
+#include <cstdio>
+#include <initializer_list>
+
+#include "fake_cuda.hpp"
+
+#include "../myrt_b200/csrc/rayorder.hpp"
+
+using namespace myrt_b200;
+
+static bool sound = true;
+static void check(bool ok, char const* what) {
+  if (!ok) std::printf("%s\n", what);
+  sound = sound && ok;
+}
+
+// One use of n slots as the library makes it; bad_launch: the kernels after the
+// count do not start, so the counts stay.
+static bool use(ray_order& o, size_t n, bool bad_launch) {
+  cudaStream_t const s = fake::stream(1);
+  if (!ensure_ray_order(o, n, s)) {
+    check(o.cap < n || !o.clean, "refused with room");
+    return false;
+  }
+  cudaError_t const e = use_ray_order(o, s, [&] {
+    bool zero = true;
+    for (size_t i = 0; i < kOrderBins; i += 61) zero = zero && o.dev.count[i] == 0;
+    check(zero, "counts left behind");
+    check(o.cap >= n && fake::memory.at(o.dev.perm) >= n * 4 && fake::memory.at(o.dev.rec) >= n * 8, "too small");
+    check(o.dev.ctr[0] == 0 && o.dev.ctr[1] == 0 && o.dev.ctr[2] == 0, "counters not zero");
+    if (bad_launch) {
+      for (size_t i = 0; i < kOrderBins; i += 61) o.dev.count[i] = 7;
+      fake::last = cudaErrorLaunchOutOfResources;
+    }
+  });
+  return e == cudaSuccess;
+}
+
+int main() {
+  int checked = 0;
+  for (size_t limit : {SIZE_MAX, size_t(34) << 20, size_t(16) << 20})
+    for (int bad = -1; bad < 5; ++bad)
+      for (int fail = -1; fail < 32; ++fail) {
+        fake::reset(fail);
+        fake::limit = limit;
+        ray_order o;
+        int k = 0, done = 0;
+        for (size_t n : {40, 1000, 1000, 70000, 33})
+          done += use(o, n, k++ == bad);
+        fake::limit = SIZE_MAX;
+        fake::fail_at = -1;
+        check(use(o, 50000, false), "no recovery");
+        if (limit == SIZE_MAX && bad < 0 && fail < 0) check(done == 5, "a sound use failed");
+        free_ray_order(o);
+        check(fake::held == 0, "memory left");
+        if (!sound) {
+          std::printf("limit %zu, bad launch %d, failing call %d\n", limit, bad, fail);
+          return 1;
+        }
+        ++checked;
+      }
+  std::printf("%d\n", checked);
+  return 0;
+}
