@@ -147,7 +147,8 @@ int order_rays(myrt_ctx* ctx, trace_args& a, int lane, cudaStream_t s) {
   }
   int rc = check_cuda(ctx, cudaStreamWaitEvent(s, o.done, 0), "ray order wait");
   if (rc) return rc;
-  if (!ensure_ray_order(o.order, a.n, s)) return MYRT_OK;
+  rc = check_cuda(ctx, ensure_ray_order(o.order, a.n, s), "ray order scratch");
+  if (rc || o.order.cap < a.n) return rc;
   batch_cell cell{a.rays, {}, {}};
   ray_cell_grid(ctx->scene.bounds, cell.lo, cell.scale);
   rc = check_cuda(ctx, build_ray_order(o.order, cell, a.n, nullptr, s), "ray order launch");

@@ -539,9 +539,10 @@ int ensure_queues(myrt_ctx* ctx, physical_state& P, size_t paths) {
 // The visiting order's scratch, which a wave can do without: taken after everything it cannot do
 // without (queues, the guide's points and lobes, tables). Without room for it the queues are visited
 // as they are.
-void ensure_queue_order(myrt_ctx* ctx, physical_state& P, size_t paths) {
+int ensure_queue_order(myrt_ctx* ctx, physical_state& P, size_t paths) {
   uint32_t const order = ctx->tuning.trace_order;
-  if (order == 2 || (order == 0 && paths >= kOrderMin)) ensure_ray_order(P.order, paths, ctx->stream);
+  if (order == 1 || (order == 0 && paths < kOrderMin)) return MYRT_OK;
+  return check_cuda(ctx, ensure_ray_order(P.order, paths, ctx->stream), "queue order scratch");
 }
 
 pt_scene scene_of(myrt_ctx const* ctx) {
@@ -894,7 +895,8 @@ int render_physical_frames(myrt_ctx* ctx, myrt_camera const* cam, myrt_render_pa
   size_t const bytes = sizeof(pt_scene) + plan.size() * sizeof(pt_job);
   rc = grow_bytes(ctx, &P.tables, P.tables_cap, bytes, "wave tables");
   if (rc) return rc;
-  ensure_queue_order(ctx, P, max_paths);
+  rc = ensure_queue_order(ctx, P, max_paths);
+  if (rc) return rc;
   std::vector<unsigned char> host(bytes);
   std::memcpy(host.data(), &sc, sizeof(pt_scene));
   for (size_t i = 0; i < plan.size(); ++i)
@@ -970,7 +972,8 @@ int build_graph(myrt_batch* b) {
     if (rc) return rc;
     b->d_jobs_cap = bytes;
   }
-  ensure_queue_order(ctx, b->queues, max_paths);
+  rc = ensure_queue_order(ctx, b->queues, max_paths);
+  if (rc) return rc;
   for (size_t w = 0; w < b->plan.size(); ++w)
     std::memcpy(b->h_jobs + w * nj, b->plan[w].jobs.data(), nj * sizeof(pt_job));
   cudaStream_t const st = ctx->stream;

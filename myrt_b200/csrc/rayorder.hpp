@@ -33,15 +33,17 @@ inline void free_ray_order(ray_order& o) {
   o = ray_order{};
 }
 
-// Room for n slots, with zero counts. False, with nothing held and no error left
-// behind, when the device has none: the caller then visits in input order.
-inline bool ensure_ray_order(ray_order& o, size_t n, cudaStream_t s) {
-  if (o.cap >= n && o.dev.perm && o.clean) return true;
-  if (cudaStreamSynchronize(s) != cudaSuccess) {
+// Room for n slots, with zero counts, where the device has it; without it
+// nothing is held, o.cap is below n and the caller visits in input order. An
+// error is a stream that cannot be waited for: work before it failed, or it is
+// being captured, when no memory may be taken.
+inline cudaError_t ensure_ray_order(ray_order& o, size_t n, cudaStream_t s) {
+  if (o.cap >= n && o.clean) return cudaSuccess;
+  if (cudaError_t const e = cudaStreamSynchronize(s); e != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return e;
   }
-  if (o.cap < n || !o.dev.perm) {
+  if (o.cap < n) {
     free_ray_order(o);
     auto alloc = [](auto** p, size_t bytes) { return cudaMalloc(reinterpret_cast<void**>(p), bytes) == cudaSuccess; };
     size_t const warps = (n + 31) / 32;
@@ -50,13 +52,12 @@ inline bool ensure_ray_order(ray_order& o, size_t n, cudaStream_t s) {
         alloc(&o.dev.ctr, 4 * sizeof(uint32_t)))
       o.cap = n;
   }
-  if (o.cap >= n && cudaMemsetAsync(o.dev.count, 0, size_t(kOrderBins) * 4, s) == cudaSuccess) {
-    o.clean = true;
-    return true;
+  o.clean = o.cap >= n && cudaMemsetAsync(o.dev.count, 0, size_t(kOrderBins) * 4, s) == cudaSuccess;
+  if (!o.clean) {
+    cudaGetLastError();
+    free_ray_order(o);
   }
-  cudaGetLastError();
-  free_ray_order(o);
-  return false;
+  return cudaSuccess;
 }
 
 // One use: launch() starts the kernels that count, turn counts into positions

@@ -833,8 +833,12 @@ int render_reference_frames(myrt_ctx* ctx, myrt_camera const* cam, myrt_render_p
   uint32_t* const shadow_count = R.counts + 2 * kMaxFramesInFlight;
   auto* const trace_pass = trace_pass_of(sd.sdf.n_drawables > 0, split_shadow);
   uint64_t const max_threads = uint64_t(K) * nb * kBlock;  // a slot per thread of a pass's grid
-  bool const can_sort = (order == 2 || (order == 0 && size_t(K) * n >= kOrderMin)) &&
-      ensure_ray_order(R.order, size_t(max_threads), ctx->stream);
+  bool can_sort = order == 2 || (order == 0 && size_t(K) * n >= kOrderMin);
+  if (can_sort) {
+    rc = check_cuda(ctx, ensure_ray_order(R.order, size_t(max_threads), ctx->stream), "pass order scratch");
+    if (rc) return rc;
+    can_sort = R.order.cap >= max_threads;
+  }
   pass_cell cell{nullptr, nullptr, uint32_t(n), nb, {}, {}};
   ray_cell_grid(ctx->scene.bounds, cell.lo, cell.scale);
   for (int f0 = 0; f0 < F; f0 += int(K)) {

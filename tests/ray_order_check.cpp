@@ -23,11 +23,18 @@ static void check(bool ok, char const* what) {
 // count do not start, so the counts stay.
 static bool use(ray_order& o, size_t n, bool bad_launch) {
   cudaStream_t const s = fake::stream(1);
-  if (!ensure_ray_order(o, n, s)) {
-    check(o.cap < n || !o.clean, "refused with room");
+  bool const fits = o.cap >= n && o.clean;
+  int const before = fake::calls;
+  cudaError_t e = ensure_ray_order(o, n, s);
+  check(!fits || fake::calls == before, "calls without need");
+  check((e != cudaSuccess) == (!fits && fake::fail_at == before), "a failed wait hidden, or an error without one");
+  check(fake::last == cudaSuccess, "an error left for the next launch check");
+  if (e != cudaSuccess) return false;
+  if (o.cap < n) {
+    check(o.cap == 0 && fake::held == 0, "no room, but memory held");
     return false;
   }
-  cudaError_t const e = use_ray_order(o, s, [&] {
+  e = use_ray_order(o, s, [&] {
     bool zero = true;
     for (size_t i = 0; i < kOrderBins; i += 61) zero = zero && o.dev.count[i] == 0;
     check(zero, "counts left behind");
