@@ -138,8 +138,8 @@ struct batch_cell {
 // The batch's visiting order (rayorder.cuh) into the lane's scratch and a.perm;
 // input order (a.perm null) when the device has no room for it. The scratch of
 // a lane is reused by later queries on any stream: each use waits for the
-// previous one.
-int order_rays(myrt_ctx* ctx, trace_args& a, int lane, cudaStream_t s) {
+// previous one. used: kernels may be using the scratch from here on.
+int order_rays(myrt_ctx* ctx, trace_args& a, int lane, cudaStream_t s, bool& used) {
   auto& o = ctx->order[lane];
   if (!o.done) {
     int rc = check_cuda(ctx, cudaEventCreateWithFlags(&o.done, cudaEventDisableTiming), "ray order event");
@@ -151,6 +151,7 @@ int order_rays(myrt_ctx* ctx, trace_args& a, int lane, cudaStream_t s) {
   if (rc || o.order.cap < a.n) return rc;
   batch_cell cell{a.rays, {}, {}};
   ray_cell_grid(ctx->scene.bounds, cell.lo, cell.scale);
+  used = true;
   rc = check_cuda(ctx, build_ray_order(o.order, cell, a.n, nullptr, s), "ray order launch");
   if (!rc) a.perm = o.order.dev.perm;
   return rc;
@@ -179,14 +180,20 @@ int launch_trace(myrt_ctx* ctx, trace_args a, int intersector, bool any, bool st
     }
     cudaEventRecord(ev[0], s);
   }
-  int rc = sorted ? order_rays(ctx, a, lane, s) : MYRT_OK;
+  bool used = false;
+  int rc = sorted ? order_rays(ctx, a, lane, s, used) : MYRT_OK;
   if (ctx->time_phases) cudaEventRecord(ev[1], s);
   if (!rc) rc = launch_trace_kernels(ctx, a, intersector, any, stats, s);
   if (ctx->time_phases) {
     cudaEventRecord(ev[2], s);
     ctx->phase_pending.push_back(ev);
   }
-  if (!rc && sorted) rc = check_cuda(ctx, cudaEventRecord(ctx->order[lane].done, s), "ray order record");
+  // the next use of the lane's scratch, on whatever stream, waits for this one: also after an error,
+  // when the order's kernels may be in flight
+  if (used) {
+    cudaError_t const e = mark_ray_order_use(ctx->order[lane].done, s);
+    if (!rc) rc = check_cuda(ctx, e, "ray order record");
+  }
   return rc;
 }
 

@@ -74,4 +74,12 @@ cudaError_t use_ray_order(ray_order& o, cudaStream_t s, LAUNCH const& launch) {
   return e != cudaSuccess ? e : l;
 }
 
+// Records the end of a use for the streams of later uses; where that fails, the
+// host waits for it instead.
+inline cudaError_t mark_ray_order_use(cudaEvent_t done, cudaStream_t s) {
+  cudaError_t const e = cudaEventRecord(done, s);
+  if (e != cudaSuccess) cudaStreamSynchronize(s);
+  return e;
+}
+
 }  // namespace myrt_b200

@@ -48,8 +48,43 @@ static bool use(ray_order& o, size_t n, bool bad_launch) {
   return e == cudaSuccess;
 }
 
+// Queries on two streams that share one scratch as api.cu's launch_trace does:
+// each waits for the one before, also when that one's traversal launch failed.
+static void shared(int bad) {
+  cudaEvent_t const done = fake::event(9);
+  ray_order o;
+  std::set<int> users;
+  for (int k = 0; k < 6; ++k) {
+    cudaStream_t const s = fake::stream(1 + k % 2);
+    if (cudaStreamWaitEvent(s, done, 0) != cudaSuccess) continue;
+    bool used = false;
+    if (ensure_ray_order(o, 100, s) == cudaSuccess && o.cap >= 100) {
+      used = true;
+      use_ray_order(o, s, [&] {
+        for (int w : users) check(fake::after[s].count(w) || fake::host.count(w), "a use beside another");
+        users.insert(fake::launch(s));
+      });
+    }
+    bool const traversal_failed = k == bad;
+    if (!traversal_failed && used) users.insert(fake::launch(s));
+    if (used) mark_ray_order_use(done, s);
+  }
+  fake::last = cudaSuccess;
+  free_ray_order(o);
+}
+
 int main() {
   int checked = 0;
+  for (int bad = -1; bad < 6; ++bad)
+    for (int fail = -1; fail < 32; ++fail) {
+      fake::reset(fail);
+      shared(bad);
+      if (!sound) {
+        std::printf("shared: bad traversal %d, failing call %d\n", bad, fail);
+        return 1;
+      }
+      ++checked;
+    }
   for (size_t limit : {SIZE_MAX, size_t(34) << 20, size_t(16) << 20})
     for (int bad = -1; bad < 5; ++bad)
       for (int fail = -1; fail < 32; ++fail) {
