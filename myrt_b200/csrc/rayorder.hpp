@@ -20,16 +20,21 @@ struct ray_order_dev {
   uint32_t* perm = nullptr;    // the order: slot of the i-th thread
   uint32_t* ctr = nullptr;     // warps taken apart, rays of the others, positions given out
 };
+// Two allocations, the cells' tables kept while the slots' part grows: a cudaMalloc costs the first
+// query of a context 0.3 ms whatever its size (and tens of ms when the host is busy). First query of
+// 1 Mi / 28 M rays, and 28 M after 1 Mi: six allocations 1.75 / 7.7 / 9.0 ms, two 1.15 / 6.7 / 6.7 ms
+// (the radix sort's five: 2.2 / 8.4 / 10.2).
 struct ray_order {
-  ray_order_dev dev;
+  ray_order_dev dev;   // count, offset and ctr in `cells`; rec, perm and warp in `slots`
+  void* cells = nullptr;
+  void* slots = nullptr;
   size_t cap = 0;      // slots
   bool clean = false;  // the counts are zero; not after a use whose launches may have run in part
 };
 
 inline void free_ray_order(ray_order& o) {
-  for (void* p : {static_cast<void*>(o.dev.count), static_cast<void*>(o.dev.offset), static_cast<void*>(o.dev.rec),
-           static_cast<void*>(o.dev.warp), static_cast<void*>(o.dev.perm), static_cast<void*>(o.dev.ctr)})
-    cudaFree(p);
+  cudaFree(o.cells);
+  cudaFree(o.slots);
   o = ray_order{};
 }
 
@@ -44,13 +49,18 @@ inline cudaError_t ensure_ray_order(ray_order& o, size_t n, cudaStream_t s) {
     return e;
   }
   if (o.cap < n) {
-    free_ray_order(o);
-    auto alloc = [](auto** p, size_t bytes) { return cudaMalloc(reinterpret_cast<void**>(p), bytes) == cudaSuccess; };
-    size_t const warps = (n + 31) / 32;
-    if (alloc(&o.dev.count, size_t(kOrderBins) * 4) && alloc(&o.dev.offset, size_t(kOrderBins) * 4) &&
-        alloc(&o.dev.rec, warps * 32 * 8) && alloc(&o.dev.warp, warps * 4) && alloc(&o.dev.perm, warps * 32 * 4) &&
-        alloc(&o.dev.ctr, 4 * sizeof(uint32_t)))
+    size_t const bins = kOrderBins, warps = (n + 31) / 32;
+    cudaFree(o.slots);
+    o.slots = nullptr;
+    o.cap = 0;
+    if ((o.cells || cudaMalloc(&o.cells, (2 * bins + 4) * 4) == cudaSuccess) &&
+        cudaMalloc(&o.slots, warps * (32 * 12 + 4)) == cudaSuccess) {
+      auto* const c = static_cast<uint32_t*>(o.cells);
+      auto* const rec = static_cast<uint2*>(o.slots);
+      auto* const perm = reinterpret_cast<uint32_t*>(rec + warps * 32);
+      o.dev = ray_order_dev{c, c + bins, rec, perm + warps * 32, perm, c + 2 * bins};
       o.cap = n;
+    }
   }
   o.clean = o.cap >= n && cudaMemsetAsync(o.dev.count, 0, size_t(kOrderBins) * 4, s) == cudaSuccess;
   if (!o.clean) {

@@ -15,7 +15,7 @@ def test_helper_survives_every_failing_call(tmp_path, check):
     if gxx is None:
         pytest.skip("g++ not available")
     exe = tmp_path / check
-    subprocess.run([gxx, "-O1", "-std=c++20", "-Wall", "-Wextra", "-Werror", "-Wno-unused-parameter", "-isystem",
+    subprocess.run([gxx, "-O2", "-std=c++20", "-Wall", "-Wextra", "-Werror", "-Wno-unused-parameter", "-isystem",
                     "/usr/local/cuda/include", "-o", str(exe), str(ROOT / "tests" / f"{check}.cpp")], check=True)
     res = subprocess.run([str(exe)], capture_output=True, text=True)
     assert res.returncode == 0, res.stdout
