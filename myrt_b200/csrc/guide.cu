@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "../../include/myrt_cuda.h"
+#include "call_buffer.hpp"
 #include "ctx.hpp"
 #include "guide.cuh"
 #include "tc.cuh"
@@ -68,8 +69,7 @@ struct guide_state {
   size_t records_cap = 0;        // in records
   float4* samples = nullptr;     // 4 float4 per sample
   size_t samples_cap = 0;
-  void* call_buf = nullptr;      // inputs and outputs of the host-array calls (call_buffer)
-  size_t call_cap = 0;
+  call_buffer call;              // inputs and outputs of the host-array calls
   myrt_guide_params prm{0.5f, 1e-2f, 16u, 16384u, 1u, 1u, 1u, 10.f, 0u, 0u};
   uint32_t wave = 0;
   uint32_t tag = 0;
@@ -880,28 +880,6 @@ template <typename T> int grow(myrt_ctx* ctx, T** p, size_t& cap, size_t want, s
   return MYRT_OK;
 }
 
-// Device memory for one host-array call (evaluation, gradients, training on
-// host samples), kept between calls: cudaMalloc and the synchronising cudaFree
-// of two buffers cost such a call about as much as its kernels. Above
-// kCallKeep bytes it goes back at the end of the call (call_release). Calls of
-// one context run one after another on its stream and wait for it.
-constexpr size_t kCallKeep = size_t(64) << 20;
-int call_buffer(myrt_ctx* ctx, guide_state& g, size_t bytes) {
-  if (g.call_cap >= bytes) return MYRT_OK;
-  cudaFree(g.call_buf);
-  g.call_buf = nullptr;
-  g.call_cap = 0;
-  int rc = check_cuda(ctx, cudaMalloc(&g.call_buf, bytes), "guide call buffer");
-  if (!rc) g.call_cap = bytes;
-  return rc;
-}
-void call_release(guide_state& g) {
-  if (g.call_cap <= kCallKeep) return;
-  cudaFree(g.call_buf);
-  g.call_buf = nullptr;
-  g.call_cap = 0;
-}
-
 int init_params(myrt_ctx* ctx, guide_state& g) {
   std::vector<float> h(kParams, 0.f);
   std::mt19937 rng(g.prm.seed);
@@ -1024,7 +1002,7 @@ void free_guide(guide_state* g) {
            static_cast<void*>(g->grads), static_cast<void*>(g->partials), static_cast<void*>(g->w_bf16),
            static_cast<void*>(g->sums),
            static_cast<void*>(g->counters), static_cast<void*>(g->points), static_cast<void*>(g->lobes),
-           static_cast<void*>(g->records), static_cast<void*>(g->samples), g->call_buf})
+           static_cast<void*>(g->records), static_cast<void*>(g->samples), g->call.p})
     cudaFree(p);
   delete g;
 }
@@ -1171,15 +1149,15 @@ int guide_eval(myrt_ctx* ctx, float const* points, uint32_t n, float* lobes) {
   if (rc || n == 0) return rc;
   guide_state& g = *ctx->guide;
   cudaStream_t st = ctx->stream;
-  rc = call_buffer(ctx, g, size_t(n) * (256 + 48));
+  rc = check_cuda(ctx, g.call.take(size_t(n) * (256 + 48)), "guide call buffer");
   if (rc) return rc;
-  auto* const d_lobes = static_cast<float4*>(g.call_buf);
+  auto* const d_lobes = static_cast<float4*>(g.call.p);
   auto* const d_pts = d_lobes + size_t(n) * 16;
   rc = check_cuda(ctx, cudaMemcpyAsync(d_pts, points, size_t(n) * 48, cudaMemcpyHostToDevice, st), "upload");
   if (!rc) rc = launch_forward(ctx, make_mlp(ctx), d_pts, nullptr, n, n, false, d_lobes, st);
   if (!rc) rc = check_cuda(ctx, cudaMemcpyAsync(lobes, d_lobes, size_t(n) * 256, cudaMemcpyDeviceToHost, st), "read");
   if (!rc) rc = check_cuda(ctx, cudaStreamSynchronize(st), "guide eval");
-  call_release(g);
+  g.call.end_call(st, rc != MYRT_OK);
   return rc;
 }
 
@@ -1188,9 +1166,9 @@ int guide_gradients(myrt_ctx* ctx, float const* samples, uint32_t n, float* grad
   if (rc) return rc;
   guide_state& g = *ctx->guide;
   cudaStream_t st = ctx->stream;
-  rc = call_buffer(ctx, g, size_t(n) * 64 + 16);
+  rc = check_cuda(ctx, g.call.take(size_t(n) * 64 + 16), "guide call buffer");
   if (rc) return rc;
-  auto* const d_s = static_cast<float4*>(g.call_buf);
+  auto* const d_s = static_cast<float4*>(g.call.p);
   auto* const d_loss = reinterpret_cast<float*>(d_s + size_t(n) * 4);
   if (n) rc = check_cuda(ctx, cudaMemcpyAsync(d_s, samples, size_t(n) * 64, cudaMemcpyHostToDevice, st), "upload");
   if (!rc) rc = check_cuda(ctx, cudaMemsetAsync(g.grads, 0, kParams * 4, st), "clear");
@@ -1217,7 +1195,7 @@ int guide_gradients(myrt_ctx* ctx, float const* samples, uint32_t n, float* grad
   if (!rc && loss) rc = check_cuda(ctx, cudaMemcpyAsync(loss, d_loss, 4, cudaMemcpyDeviceToHost, st), "read");
   if (!rc) rc = check_cuda(ctx, cudaMemsetAsync(g.grads, 0, kParams * 4, st), "clear");
   if (!rc) rc = check_cuda(ctx, cudaStreamSynchronize(st), "guide gradients");
-  call_release(g);
+  g.call.end_call(st, rc != MYRT_OK);
   return rc;
 }
 
@@ -1226,9 +1204,9 @@ int guide_train_samples(myrt_ctx* ctx, float const* samples, uint32_t n, uint32_
   if (rc) return rc;
   guide_state& g = *ctx->guide;
   cudaStream_t st = ctx->stream;
-  rc = call_buffer(ctx, g, size_t(n) * 64 + std::max<size_t>(steps, 1) * 4);
+  rc = check_cuda(ctx, g.call.take(size_t(n) * 64 + std::max<size_t>(steps, 1) * 4), "guide call buffer");
   if (rc) return rc;
-  auto* const d_s = static_cast<float4*>(g.call_buf);
+  auto* const d_s = static_cast<float4*>(g.call.p);
   auto* const d_loss = reinterpret_cast<float*>(d_s + size_t(n) * 4);
   if (n) rc = check_cuda(ctx, cudaMemcpyAsync(d_s, samples, size_t(n) * 64, cudaMemcpyHostToDevice, st), "upload");
   if (!rc) rc = check_cuda(ctx, cudaMemsetAsync(d_loss, 0, std::max<size_t>(steps, 1) * 4, st), "clear");
@@ -1251,7 +1229,7 @@ int guide_train_samples(myrt_ctx* ctx, float const* samples, uint32_t n, uint32_
   if (!rc && loss_per_step && steps)
     rc = check_cuda(ctx, cudaMemcpyAsync(loss_per_step, d_loss, size_t(steps) * 4, cudaMemcpyDeviceToHost, st), "read");
   if (!rc) rc = check_cuda(ctx, cudaStreamSynchronize(st), "guide training");
-  call_release(g);
+  g.call.end_call(st, rc != MYRT_OK);
   return rc;
 }
 

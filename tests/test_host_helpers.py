@@ -9,7 +9,7 @@ import pytest
 ROOT = Path(__file__).resolve().parent.parent
 
 
-@pytest.mark.parametrize("check", ["stream_fork_check", "ray_order_check"])
+@pytest.mark.parametrize("check", ["stream_fork_check", "ray_order_check", "call_buffer_check"])
 def test_helper_survives_every_failing_call(tmp_path, check):
     gxx = shutil.which("g++")
     if gxx is None:
