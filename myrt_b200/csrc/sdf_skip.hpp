@@ -204,8 +204,11 @@ struct sdf_cells {
   std::vector<int4> outer;     // 2 per program: (lo.xyz, 1 / cell) bits; (nx, ny, nz, first cell), nx = 0: none
 };
 
-// cells_long: cells along the grid's longest axis (2..128).
-inline void sdf_cell_tables(myrt_sdf_view const* v, int cells_long, sdf_cells& out) {
+// cells_long: cells along the grid's longest axis (2..128). max_entries: segments that all programs'
+// first grids may hold together; the second grids, which only folds have and evaluation can do
+// without, hold at most half as many and take nothing from them.
+inline void sdf_cell_tables(
+    myrt_sdf_view const* v, int cells_long, sdf_cells& out, size_t max_entries = size_t(1) << 26) {
   out = sdf_cells{};
   out.hdr.assign(3 * v->program_count, make_int4(0, 0, 0, 0));
   out.outer.assign(2 * v->program_count, make_int4(0, 0, 0, 0));
@@ -217,7 +220,7 @@ inline void sdf_cell_tables(myrt_sdf_view const* v, int cells_long, sdf_cells& o
     double k = 0.0, delta = 0.0;
   };
   bool any = false;
-  size_t const max_entries = size_t(1) << 26;
+  size_t outer_entries = 0;  // of out.list
   for (size_t p = 0; p < v->program_count; ++p) {
     myrt_sdf_program const pr = v->programs[p];
     if (pr.count >= 65536) continue;
@@ -302,10 +305,10 @@ inline void sdf_cell_tables(myrt_sdf_view const* v, int cells_long, sdf_cells& o
       dims[a] = std::max(1, std::min(n_long, int(std::ceil((hi[a] - double(lo_f[a])) * double(inv_f)))));
     }
     // Appends the cell lists of one grid to out.start / out.list. False when
-    // they would take too many entries.
+    // they would take more than `room` entries.
     // z-slabs of cells on host threads; each keeps its cells' segment counts
     // and segments, concatenated in cell order afterwards
-    auto add_grid = [&](float const (&lo_f)[3], float inv_f, int const (&dims)[3], double scale) -> bool {
+    auto add_grid = [&](float const (&lo_f)[3], float inv_f, int const (&dims)[3], double scale, size_t room) -> bool {
       size_t const ncell = size_t(dims[0]) * dims[1] * dims[2];
       double const cell = 1.0 / double(inv_f);
       // the device finds a point's cell by rounded float arithmetic: widen each
@@ -401,11 +404,11 @@ inline void sdf_cell_tables(myrt_sdf_view const* v, int cells_long, sdf_cells& o
         fill(0);
         for (std::thread& th : pool) th.join();
       }
-      size_t total = out.list.size();
-      for (slab const& sl : slabs) total += sl.segs.size();
-      if (total > max_entries) return false;
+      size_t entries = 0;
+      for (slab const& sl : slabs) entries += sl.segs.size();
+      if (entries > room) return false;
       out.start.reserve(first_start + ncell + 1);
-      out.list.reserve(total);
+      out.list.reserve(first_entry + entries);
       for (slab const& sl : slabs) {
         for (int n_seg : sl.sizes) {
           out.start.push_back(int(out.list.size()));
@@ -423,7 +426,8 @@ inline void sdf_cell_tables(myrt_sdf_view const* v, int cells_long, sdf_cells& o
       return true;
     };
     size_t const first_start = out.start.size();
-    if (!add_grid(lo_f, inv_f, dims, scale)) continue;  // too large: no cells for this program
+    size_t const inner = out.list.size() - outer_entries;
+    if (!add_grid(lo_f, inv_f, dims, scale, max_entries - inner)) continue;  // too large: no cells for this program
     double const margin = 2e-3 + 4e-6 * double(n_prims) * scale;
     // escape sphere about the grid's centre; the radius carries a relative
     // margin for the rounding of values and positions far from the field
@@ -458,7 +462,9 @@ inline void sdf_cell_tables(myrt_sdf_view const* v, int cells_long, sdf_cells& o
       scale2 = std::fmax(scale2, std::fabs(mid) + 2.0 * half + 4.0 / double(inv_f));
     }
     size_t const outer_start = out.start.size();
-    if (!add_grid(lo2, inv2, dims2, scale2)) continue;
+    size_t const before = out.list.size();
+    if (!add_grid(lo2, inv2, dims2, scale2, max_entries / 2 - outer_entries)) continue;
+    outer_entries += out.list.size() - before;
     int lo2_bits[3], inv2_bits;
     std::memcpy(lo2_bits, lo2, sizeof lo2_bits);
     std::memcpy(&inv2_bits, &inv2, sizeof inv2_bits);
