@@ -273,7 +273,10 @@ int myrt_trace_any_device(myrt_ctx* ctx, const myrt_ray* rays, uint32_t n, uint8
  * nodes[i] = wide nodes fetched, tris[i] = triangles tested. Used to count the
  * algorithmic bytes per ray (80 B per node, 48 B per triangle). The counted walk
  * tests child boxes at exactly their quantised planes; the queries widen each
- * plane by 1/64 of a quantum (trace.cuh), so they may fetch a few more nodes. */
+ * plane by 1/64 of a quantum (trace.cuh), so they may fetch a few more nodes, and
+ * where the float triangle test accepts a ray that passes just outside a
+ * triangle's box (triangles of 1e-5 and less), they may report that hit where
+ * the counted walk does not. */
 int myrt_trace_closest_stats_device(myrt_ctx* ctx, const myrt_ray* rays, uint32_t n, myrt_hit* hits,
     uint32_t* nodes, uint32_t* tris, int intersector, void* stream);
 
