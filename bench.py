@@ -1142,7 +1142,7 @@ def run_sdf_workload(args, emit: bool = True):
          "sdf_shape": args.sdf_shape},
         {"mrays_per_s": rays / (ms / 1e3) / 1e6, "rays_per_sample": rays / samples,
          f"rel_rmse_vs_fp64_{oracle_spp}spp": err, "rel_rmse_spp": spp * args.steps,
-         "fp32_roofline": _sdf_fp32_roofline(),
+         "fp32_roofline": _sdf_fp32_roofline(compiled=args.sdf_shape == "chain" and args.sdf_cells != 1),
          "e2e": {"value": samples / e2e_s, "unit": "samples/s", "h2d_bytes_per_step": 128,
                  "d2h_bytes_per_step": W * H * 16, "api": "myrt_render + myrt_read_accumulation"},
          "clocks": clocks.summary()})
@@ -1152,20 +1152,21 @@ def run_sdf_workload(args, emit: bool = True):
     return 0
 
 
-def _sdf_fp32_roofline():
+def _sdf_fp32_roofline(compiled):
     """FP32 roofline of the SDF extend kernel: the ncu-counted FP32 FLOP rate of
     one launch (profiles/sdf_hybrid_extend.md) against the nominal FP32 peak at
-    the maximum SM clock (148 SMs x 128 lanes x 2 FLOPs)."""
-    achieved = profiled_sdf_fp32_tflops()
+    the maximum SM clock (148 SMs x 128 lanes x 2 FLOPs). The count is of a left
+    fold's compiled records; a field that the interpreter evaluates has none."""
+    achieved = profiled_sdf_fp32_tflops() if compiled else None
     peaks, _ = measured_peaks()
     mhz = float(peaks.get("sm_max_mhz", 1965.0))
     peak = 148 * 128 * 2 * mhz * 1e6 / 1e12
     return {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak if achieved else None,
-            "source": "ncu FP32 thread-instruction counts of k_pt_extend<1> as an interpreter (one launch, 1 Mi "
-                      "camera rays), before left folds were compiled into records; peak "
-                      "nominal at sm_max_mhz; the evaluator runs without FMA contraction (bit-exact with the "
-                      "reference's march) and is bound by divergent issue, not FP32 throughput"}
+            "source": ("ncu FP32 thread-instruction counts of k_pt_extend<1> on the compiled left fold (one launch, "
+                       "1 Mi camera rays)" if compiled else "no count of this field's kernel")
+                      + "; peak nominal at sm_max_mhz; the evaluator rounds as the reference's march (bit-exact) and "
+                        "is bound by divergent issue, not FP32 throughput"}
 
 
 def run_post_workload(args):
