@@ -144,7 +144,8 @@ typedef struct myrt_tuning {
   uint32_t refill;           /* persistent: refill once at least this many lanes of a warp are idle (1..32) */
   uint32_t blocks_per_sm;    /* persistent: resident 128-thread blocks per SM (0 = occupancy maximum) */
   uint32_t trace_min_blocks; /* one-thread-per-ray: register cap as blocks per SM: 8 (64 regs; 0 = 8),
-                                10 (48 regs), 12 */
+                                10 (48 regs), 12; both slower wherever measured (27.9 M closest hits 7
+                                and 18 %), kept to measure other scenes */
   uint32_t trace_unit_steps; /* one-thread-per-ray: 0 = a node and all its triangles per iteration,
                                 1 = one node, triangle or pop per iteration */
   uint32_t wave_paths;       /* physical / guided wavefront: paths in flight per wave (0 = 16 Mi; 4 Mi
@@ -196,8 +197,8 @@ typedef struct myrt_tuning {
                                 2 = one thread per queue entry (the grid covers the wave's paths
                                 up to 16 times the blocks the device holds, which then walk over
                                 the rest; the mesh traversal kernels run at 64 registers, or under a
-                                48-register cap when
-                                pt_blocks_per_sm is 10 or more).
+                                48-register cap when pt_blocks_per_sm is 10 or more, 4 % slower on a
+                                64-spp frame).
                                 Results never depend on it. */
   uint32_t ref_frames;       /* reference shading (myrt_render): frames of one call whose passes run
                                 together, each in its own region of ray slots (0 = as many as fill
