@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <functional>
 #include <thread>
 #include <vector>
 
@@ -204,6 +205,18 @@ struct sdf_cells {
   std::vector<int4> outer;     // 2 per program: (lo.xyz, 1 / cell) bits; (nx, ny, nz, first cell), nx = 0: none
 };
 
+// As many host threads as there are cores, at most n (and one): n counts pieces of work of a few
+// hundred microseconds, since starting 16 threads takes 0.2 ms.
+inline int host_threads(size_t n) {
+  return int(std::max<size_t>(1, std::min<size_t>(n, std::thread::hardware_concurrency())));
+}
+template <class F> inline void on_threads(int n, F const& f) {  // f(0) .. f(n - 1)
+  std::vector<std::thread> pool;
+  for (int t = 1; t < n; ++t) pool.emplace_back(std::cref(f), t);
+  f(0);
+  for (std::thread& th : pool) th.join();
+}
+
 // cells_long: cells along the grid's longest axis (2..128). max_entries: segments that all programs'
 // first grids may hold together; the second grids, which only folds have and evaluation can do
 // without, hold at most half as many and take nothing from them.
@@ -322,8 +335,11 @@ inline void sdf_cell_tables(
         std::vector<int> sizes;
         std::vector<uint32_t> segs;
       };
-      int const n_threads = std::max(1, std::min<int>(dims[2], int(std::thread::hardware_concurrency())));
+      int const n_threads = host_threads(std::min(size_t(dims[2]), 1 + ncell * ns.size() / (1 << 14)));
       std::vector<slab> slabs(n_threads);
+      // the bounds are finite, and std::fmax / std::fmin are calls into the library: 2.5-3 times as long
+      auto const max = [](double a, double b) { return a > b ? a : b; };
+      auto const min = [](double a, double b) { return a < b ? a : b; };
       auto fill = [&](int t) {
         slab& out_t = slabs[t];
         std::vector<double> lb(ns.size()), ub(ns.size());
@@ -356,8 +372,8 @@ inline void sdf_cell_tables(
                 if (n.a < 0) {
                   double n2 = 0.0, f2 = 0.0;
                   for (int a = 0; a < 3; ++a) {
-                    double const o = std::fmax(0.0, std::fmax(bmin[a] - n.c[a], n.c[a] - bmax[a]));
-                    double const f = std::fmax(std::fabs(n.c[a] - bmin[a]), std::fabs(n.c[a] - bmax[a]));
+                    double const o = max(0.0, max(bmin[a] - n.c[a], n.c[a] - bmax[a]));
+                    double const f = max(std::fabs(n.c[a] - bmin[a]), std::fabs(n.c[a] - bmax[a]));
                     n2 += o * o;
                     f2 += f * f;
                   }
@@ -366,8 +382,8 @@ inline void sdf_cell_tables(
                 } else {
                   // lb of an operator node is (its primitives' smallest bound -
                   // its delta); lb + delta recovers the primitives' bound
-                  lb[i] = std::fmin(lb[n.a] + ns[n.a].delta, lb[n.b] + ns[n.b].delta) - n.delta;
-                  ub[i] = std::fmin(ub[n.a], ub[n.b]);
+                  lb[i] = min(lb[n.a] + ns[n.a].delta, lb[n.b] + ns[n.b].delta) - n.delta;
+                  ub[i] = min(ub[n.a], ub[n.b]);
                 }
               }
               open = false;
@@ -398,12 +414,7 @@ inline void sdf_cell_tables(
               out_t.sizes.push_back(int(out_t.segs.size() - before));
             }
       };
-      {
-        std::vector<std::thread> pool;
-        for (int t = 1; t < n_threads; ++t) pool.emplace_back(fill, t);
-        fill(0);
-        for (std::thread& th : pool) th.join();
-      }
+      on_threads(n_threads, fill);
       size_t entries = 0;
       for (slab const& sl : slabs) entries += sl.segs.size();
       if (entries > room) return false;
@@ -508,6 +519,7 @@ inline void sdf_chain_tables(myrt_sdf_view const* v, sdf_cells const& cells, sdf
     myrt_sdf_program const pr = v->programs[p];
     std::vector<float4> rec;
     std::vector<int> group(pr.count, -1);    // instruction -> its group
+    std::vector<int> group_end;              // group -> the instruction after its last
     std::vector<uint8_t> is_op(pr.count, 0);
     bool ok = true;
     int g = 0;
@@ -535,6 +547,7 @@ inline void sdf_chain_tables(myrt_sdf_view const* v, sdf_cells const& cells, sdf
         is_op[j] = 1;
         group[j++] = g;
       }
+      group_end.push_back(j);
       float const Rf = float(R) + 1e-6f * float(std::fabs(R));
       rec.push_back(make_float4(float(c[0]), float(c[1]), float(c[2]), Rf + k));
       rec.push_back(make_float4(off[0], off[1], off[2], bits(kind)));
@@ -542,46 +555,63 @@ inline void sdf_chain_tables(myrt_sdf_view const* v, sdf_cells const& cells, sdf
       rec.push_back(make_float4(q[0], in.op == MYRT_SDF_SPHERE ? 0.f : q[1], box ? q[2] : 0.f, k));
     }
     if (!ok || g < 2 || g >= 65535) continue;
-    // the cells' groups (both grids), and every group as one more list
-    std::vector<uint16_t> list;
-    auto close = [&] {
-      while (list.size() & 3u) list.push_back(uint16_t(g));
-    };
-    int const base = int(out.list.size() / 4);
-    for (int4 const grid : {dims, cells.outer[2 * p + 1]}) {
-      size_t const ncell = size_t(grid.x) * grid.y * grid.z;
-      for (size_t c = 0; ok && c < ncell; ++c) {
-        out.start[grid.w + c] = base + int(list.size() / 4);
-        int last = -1;
-        for (int e = cells.start[grid.w + c]; ok && e < cells.start[grid.w + c + 1]; ++e) {
-          int const s0 = int(cells.list[e] & 0xffffu), s1 = int(cells.list[e] >> 16);
-          for (int j = s0; j < s1; ++j) {
-            if (is_op[j]) {
-              ok = ok && group[j] == last;  // an operator follows its own group's primitive
-              continue;
-            }
-            if (group[j] == last) continue;  // translation, then primitive
-            // a group after the list's first needs its operator in the same segment
-            bool const first_of_list = last < 0;
-            last = group[j];
-            int end = j;
-            while (end < s1 && group[end] == last) ++end;
-            ok = ok && first_of_list != bool(is_op[end - 1]);
-            list.push_back(uint16_t(last));
-          }
-        }
-        ok = ok && last >= 0;
-        close();
+    // the cells' groups (both grids, one after the other), and every group as
+    // one more list: counted, then written where they belong, on host threads
+    int4 const grid2 = cells.outer[2 * p + 1];
+    size_t const n1 = size_t(dims.x) * dims.y * dims.z, n2 = size_t(grid2.x) * grid2.y * grid2.z, ncell = n1 + n2;
+    auto cell = [&](size_t i) { return i < n1 ? size_t(dims.w) + i : size_t(grid2.w) + (i - n1); };
+    // calls f(first, last) for the groups of each of a cell's segments; false when they are not whole groups
+    auto groups = [&](size_t c, auto const& f) {
+      int last = -1;
+      for (int e = cells.start[c]; e < cells.start[c + 1]; ++e) {
+        int j = int(cells.list[e] & 0xffffu);
+        int const end = int(cells.list[e] >> 16);
+        while (j < end && group[j] == last) ++j;  // the operator of the segment before's last group
+        if (j == end) continue;
+        // an operator follows its own group's primitive, and a group after the list's first needs its
+        // operator in the same segment, as those inside a segment have it
+        int const g0 = group[j], g1 = group[end - 1];
+        bool const first_op = is_op[std::min(end, group_end[g0]) - 1];
+        if (is_op[j] || (last < 0) == first_op || (g1 > g0 && !is_op[end - 1])) return false;
+        f(g0, g1);
+        last = g1;
       }
-      if (ncell) out.start[grid.w + ncell] = base + int(list.size() / 4);
+      return last >= 0;
+    };
+    size_t const segments = size_t(cells.start[dims.w + n1] - cells.start[dims.w]);
+    int const n_count = host_threads(segments / (1 << 15));
+    std::vector<int> batches(ncell);
+    std::vector<uint8_t> whole(n_count, 1);
+    on_threads(n_count, [&](int t) {
+      for (size_t i = ncell * t / n_count; whole[t] && i < ncell * (t + 1) / n_count; ++i) {
+        int n = 0;
+        whole[t] = groups(cell(i), [&](int g0, int g1) { n += g1 - g0 + 1; });
+        batches[i] = (n + 3) / 4;
+      }
+    });
+    size_t entries = 0;
+    for (int n : batches) entries += size_t(n);
+    for (uint8_t w : whole) ok = ok && w;
+    if (!ok || entries + out.list.size() / 4 > (size_t(1) << 28)) continue;
+    int at = int(out.list.size() / 4);
+    for (size_t i = 0; i < ncell; ++i) {
+      out.start[cell(i)] = at;
+      at += batches[i];
+      if (i + 1 == n1) out.start[dims.w + n1] = at;
     }
-    if (!ok || list.size() / 4 + out.list.size() / 4 > (size_t(1) << 28)) continue;
-    out.list.insert(out.list.end(), list.begin(), list.end());
-    list.clear();
-    for (int k = 0; k < g; ++k) list.push_back(uint16_t(k));
-    close();
-    int const full = int(out.list.size() / 4);
-    out.list.insert(out.list.end(), list.begin(), list.end());
+    if (n2) out.start[grid2.w + n2] = at;
+    int const full = at;
+    out.list.resize(4 * (size_t(full) + size_t(g + 3) / 4), uint16_t(g));  // fills lists up
+    int const n_fill = host_threads(entries / (1 << 14));
+    on_threads(n_fill, [&](int t) {
+      for (size_t i = ncell * t / n_fill; i < ncell * (t + 1) / n_fill; ++i) {
+        uint16_t* to = out.list.data() + 4 * size_t(out.start[cell(i)]);
+        groups(cell(i), [&](int g0, int g1) {
+          for (int k = g0; k <= g1; ++k) *to++ = uint16_t(k);
+        });
+      }
+    });
+    for (int k = 0; k < g; ++k) out.list[4 * size_t(full) + k] = uint16_t(k);
     out.hdr[p] = make_int4(int(out.rec.size() / 3), g, full, int(out.list.size() / 4));
     rec.push_back(make_float4(0.f, 0.f, 0.f, -HUGE_VALF));
     rec.push_back(make_float4(0.f, 0.f, 0.f, bits(MYRT_SDF_SPHERE)));
